@@ -839,13 +839,6 @@ class TissueKernel(object):
             raise ValueError('Could not order the state updates.')
         self._inter_names = [self._name(v) for v in self.inter_log]
 
-        if self.traj:
-            # The adjoint's forward pass records the states at t of every
-            # step of the launch: traj[k][state][pitch]
-            for i, st in enumerate(self.states):
-                loads.append(
-                    f'{tab}((Real *)a.traj)[((long long)k * {self.n_state}'
-                    f' + {i}) * pitch + cid] = {self._name(st)};')
 
         # Logging: states and idiff right after the loads, intermediaries
         # at the end (item ids as in include/mkg_tissue.h).
@@ -856,6 +849,16 @@ class TissueKernel(object):
         log_a = _LOG_BLOCK.format(
             cond=f'item <= {self.n_state}',
             cases=('\n' + t2 + '        ').join(cases))
+        if self.traj:
+            # The adjoint's forward pass records the states at t of every
+            # step of the launch: traj[k][state][pitch]. Written with the
+            # logged values, so by the lanes that hold a cell only: staged
+            # tiles are read by every lane, and a lane past the end of a row
+            # would write into the next row's cells
+            log_a = '\n'.join(
+                f'{tab}((Real *)a.traj)[((long long)k * {self.n_state}'
+                f' + {i}) * pitch + cid] = {self._name(st)};'
+                for i, st in enumerate(self.states)) + log_a
         first = self._name(self.states[0])
         log_a += (
             f'\n{tab}if (row >= 0 && a.nan_check && cid == 0 && '
