@@ -253,14 +253,18 @@ class AdjointKernel(object):
             if s in fwd.rl_states:
                 inf, tau = fwd.rl_states[s]
                 ri, rt = ref(inf), ref(tau)
-                seeds.append(f'{tab}  const Real E_ = {expf}(-dt_ / {rt});')
+                arg = f'-dt_ / {rt}' if self.single else \
+                    f'mkg_div(-dt_, {rt})'
+                seeds.append(f'{tab}  const Real E_ = {expf}({arg});')
                 seeds.append(f'{tab}  {A(n)} += l_ * E_;')
                 if myokit.Name(inf) not in fwd.literal_subst:
                     seeds.append(f'{tab}  {A(name(inf))} += l_ * (1 - E_);')
                 if myokit.Name(tau) not in fwd.literal_subst:
-                    seeds.append(
-                        f'{tab}  {A(name(tau))} += -l_ * ({ri} - {n}) * E_'
-                        f' * dt_ / ({rt} * {rt});')
+                    num = f'-l_ * ({ri} - {n}) * E_ * dt_'
+                    den = f'{rt} * {rt}'
+                    q = f'{num} / ({den})' if self.single else \
+                        f'mkg_div({num}, {den})'
+                    seeds.append(f'{tab}  {A(name(tau))} += {q};')
             else:
                 seeds.append(f'{tab}  {A(n)} += l_;')
                 seeds.append(f'{tab}  {A(name(s.lhs()))} += l_ * dt_;')

@@ -66,6 +66,38 @@ def _fmt_number(x, single):
     return s + 'f' if single else s
 
 
+def _reciprocal_digits(x):
+    """
+    2^32 / (the significand of a normal ``x``, in [1, 2)), rounded down and
+    below 2^32: the divisor's part of mkg_div_by, for literal divisors.
+    """
+    if not np.isfinite(x) or abs(x) < 2.0 ** -1022:
+        return None
+    return min((1 << 53) * (1 << 32) // int(abs(np.frexp(x)[0]) * (1 << 54)),
+               (1 << 32) - 1)
+
+
+def _exp_table():
+    """The table of mkg_exp: e^(j/256) in units of 2^-62, j = 0 .. 178."""
+    from decimal import Decimal, localcontext
+    with localcontext() as c:
+        c.prec = 40
+        v = [int((Decimal(j) / 256).exp() * 2**62 + Decimal('0.5'))
+             for j in range(179)]
+    return ('static __device__ const unsigned long long mkg_exp_tab[179] = {'
+            + ', '.join('0x%xull' % x for x in v) + '};')
+
+
+_MATH64 = []
+
+
+def _math64():
+    """Text of the integer exp and division of double precision kernels."""
+    if not _MATH64:
+        _MATH64.append(_exp_table() + '\n' + _read('mkg_math64.h'))
+    return _MATH64[0]
+
+
 class CudaExpressionWriter(CBasedExpressionWriter):
     """
     Writes myokit expressions as CUDA C++ for one precision.
@@ -76,14 +108,29 @@ class CudaExpressionWriter(CBasedExpressionWriter):
     counterpart of OpenCL's ``native_*`` functions
     (``myokit/formats/opencl/_ewriter.py:59-93``).
     """
-    def __init__(self, single, native_math=False, fast_divide=False):
+    def __init__(self, single, native_math=False, fast_divide=False,
+                 soft=False):
         super().__init__()
         self._single = bool(single)
         self._native = bool(native_math) and self._single
         self._fast_div = bool(fast_divide) and self._single
+        # Double precision exp and division in integer arithmetic
+        # (csrc/mkg_math64.h)
+        self._soft = bool(soft) and not self._single
         self.int_powers = set()
 
+    def divide(self, a, b):
+        """The quotient of two expressions given as text."""
+        return f'mkg_div({a}, {b})' if self._soft else f'({a}) / ({b})'
+
     def _ex_divide(self, e):
+        if self._soft:
+            num, den = self.ex(e[0]), e[1]
+            if isinstance(den, myokit.Number):
+                y = _reciprocal_digits(float(den.eval()))
+                if y is not None:
+                    return f'mkg_div_by({num}, {self.ex(den)}, {y}u)'
+            return f'mkg_div({num}, {self.ex(den)})'
         if not self._fast_div:
             return super()._ex_divide(e)
         # Single precision fast division: a constant denominator becomes a
@@ -99,7 +146,7 @@ class CudaExpressionWriter(CBasedExpressionWriter):
 
     def _fn(self, name):
         if not self._single:
-            return name
+            return 'mkg_exp' if self._soft and name == 'exp' else name
         if self._native and name in ('exp', 'log', 'sin', 'cos', 'tan',
                                      'log10'):
             return '__' + name + 'f'
@@ -152,7 +199,8 @@ class CudaExpressionWriter(CBasedExpressionWriter):
         f = self._fn('log')
         if len(e) == 1:
             return self._ex_function(e, f)
-        return f'({f}({self.ex(e[0])}) / {f}({self.ex(e[1])}))'
+        a, b = f'{f}({self.ex(e[0])})', f'{f}({self.ex(e[1])})'
+        return self.divide(a, b) if self._soft else f'({a} / {b})'
 
     def _ex_log10(self, e):
         return self._ex_function(e, self._fn('log10'))
@@ -332,8 +380,7 @@ def _pow_helpers(single):
     sq = 'sqrtf' if single else 'sqrt'
     out.append('static __device__ __forceinline__ Real mkg_pow1p5(Real x)'
                f' {{ return x * {sq}(x); }}')
-    if single:
-        out.append(_CUBIC_HELPER)
+    out.append(_CUBIC_HELPER if single else _math64())
     return '\n'.join(out)
 
 
@@ -602,7 +649,7 @@ class TissueKernel(object):
     def _generate(self):
         m = self.model
         w = CudaExpressionWriter(self.single, self.native_math,
-                                 self.math == 'fast')
+                                 self.math == 'fast', soft=True)
         w.set_lhs_function(self._name)
         real = 'float' if self.single else 'double'
         prec = myokit.SINGLE_PRECISION if self.single else \
@@ -757,7 +804,9 @@ class TissueKernel(object):
                     if myokit.Name(v) not in literal_subst)
                 inf, tau = ref(inf), ref(tau)
                 expf = w._fn('exp')
-                upd = f'{inf} - ({inf} - {n}) * {expf}(-dt_ / {tau})'
+                x = f'mkg_div(-dt_, {tau})' if not self.single else \
+                    f'-dt_ / {tau}'
+                upd = f'{inf} - ({inf} - {n}) * {expf}({x})'
                 text = f'{tab}{target} = {upd};'
                 self._upd_expr[i] = (target, upd)
                 self.census.arith += 4
