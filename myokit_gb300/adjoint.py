@@ -243,7 +243,6 @@ class AdjointKernel(object):
 
         # Seeds: lambda_{k+1} through the update of each state
         seeds = list(acc)
-        expf = w._fn('exp')
         for i, s in enumerate(states):
             lam = f'lam[(long long){i} * pitch + cid]'
             if i == fwd.i_vm:
@@ -253,12 +252,12 @@ class AdjointKernel(object):
             if s in fwd.rl_states:
                 inf, tau = fwd.rl_states[s]
                 ri, rt = ref(inf), ref(tau)
-                arg = f'-dt_ / {rt}' if self.single else \
-                    f'mkg_div(-dt_, {rt})'
-                seeds.append(f'{tab}  const Real E_ = {expf}({arg});')
-                seeds.append(f'{tab}  {A(n)} += l_ * E_;')
+                seeds.append(f'{tab}  const Real E_ = '
+                             f'{fwd.decay(tau, rt, fwd.rates)};')
+                seeds.append(f'{tab}  {A(n)} = {w.fma("l_", "E_", A(n))};')
                 if myokit.Name(inf) not in fwd.literal_subst:
-                    seeds.append(f'{tab}  {A(name(inf))} += l_ * (1 - E_);')
+                    a = A(name(inf))
+                    seeds.append(f'{tab}  {a} = {w.fma("l_", "1 - E_", a)};')
                 if myokit.Name(tau) not in fwd.literal_subst:
                     num = f'-l_ * ({ri} - {n}) * E_ * dt_'
                     den = f'{rt} * {rt}'
@@ -267,7 +266,8 @@ class AdjointKernel(object):
                     seeds.append(f'{tab}  {A(name(tau))} += {q};')
             else:
                 seeds.append(f'{tab}  {A(n)} += l_;')
-                seeds.append(f'{tab}  {A(name(s.lhs()))} += l_ * dt_;')
+                a = A(name(s.lhs()))
+                seeds.append(f'{tab}  {a} = {w.fma("l_", "dt_", a)};')
             seeds.append(f'{tab}}}')
 
         # Reverse sweep: equations in reverse evaluation order
@@ -283,13 +283,15 @@ class AdjointKernel(object):
                 # with g = 3x^2 + 2bx + c
                 x = name(lhs)
                 b, c, d = bcd
-                terms.append(f'{tab}    const Real g_ = (3 * {x} + 2 * {b})'
-                             f' * {x} + {c};')
+                g = w.fma(w.fma('2', b, f'3 * {x}'), x, c)
+                terms.append(f'{tab}    const Real g_ = {g};')
                 terms.append(f'{tab}    const Real r_ = (g_ != 0) ? a_ / g_'
                              ' : (Real)0;')
                 for rn, dx in ((b, f'{x} * {x}'), (c, x), (d, '1')):
                     if rn in valid:
-                        terms.append(f'{tab}    {A(rn)} -= r_ * ({dx});')
+                        a = A(rn)
+                        terms.append(
+                            f'{tab}    {a} = {w.fma("-r_", dx, a)};')
                 rhs = myokit.Number(0)   # no further terms
             for r in _references(rhs):
                 rn = name(r)
@@ -300,7 +302,8 @@ class AdjointKernel(object):
                 dp = local_partial(rhs, r)
                 if dp is None:
                     continue
-                terms.append(f'{tab}    {A(rn)} += a_ * ({w.ex(dp)});')
+                terms.append(f'{tab}    {A(rn)} = '
+                             f'{w.fma("a_", w.ex(dp), A(rn))};')
             if terms:
                 # With guards an equation whose adjoint is still zero is
                 # skipped; without, the sweep is straight-line code
@@ -319,7 +322,7 @@ class AdjointKernel(object):
                 dp = local_partial(rhs, r)
                 if dp is None:
                     continue
-                rev.append(f'{tab}{A(rn)} += {a} * ({w.ex(dp)});')
+                rev.append(f'{tab}{A(rn)} = {w.fma(a, w.ex(dp), A(rn))};')
 
         # Outputs
         out = []

@@ -109,7 +109,7 @@ class CudaExpressionWriter(CBasedExpressionWriter):
     (``myokit/formats/opencl/_ewriter.py:59-93``).
     """
     def __init__(self, single, native_math=False, fast_divide=False,
-                 soft=False):
+                 soft=False, fuse=False):
         super().__init__()
         self._single = bool(single)
         self._native = bool(native_math) and self._single
@@ -117,7 +117,91 @@ class CudaExpressionWriter(CBasedExpressionWriter):
         # Double precision exp and division in integer arithmetic
         # (csrc/mkg_math64.h)
         self._soft = bool(soft) and not self._single
+        # Multiply-adds and the scaling of single precision exponentials
+        # written out (see ex)
+        self._fuse = bool(fuse)
         self.int_powers = set()
+
+    # Kernels are compiled without the compiler's own contraction of
+    # multiply-adds, which depends on the code around an expression: the
+    # same equation then gives the same bits in every kernel that holds it
+    # (staged or not, whole tiles or shared ones). The multiply-adds are
+    # chosen here instead, from the expression alone.
+
+    def ex(self, e):
+        if self._fuse:
+            if isinstance(e, (myokit.Plus, myokit.Minus)):
+                return self._sum(e)
+            if isinstance(e, myokit.Exp) and self._single and \
+                    not self._native:
+                return self._scaled_exp(e[0])
+        return super().ex(e)
+
+    def fma(self, a, b, c):
+        """a * b + c, rounded once, of expressions given as text."""
+        return f'{"fmaf" if self._single else "fma"}({a}, {b}, {c})'
+
+    def _product(self, e):
+        """Two factors (text) if ``e`` is a product, or None."""
+        if isinstance(e, myokit.PrefixMinus):
+            p = self._product(e[0])
+            return p and (f'-({p[0]})', p[1])
+        if isinstance(e, myokit.Multiply):
+            return self.ex(e[0]), self.ex(e[1])
+        if isinstance(e, myokit.Power) and isinstance(e[1], myokit.Number) \
+                and float(e[1].eval()) == 2:
+            x = self.ex(e[0])
+            return x, x
+        if isinstance(e, myokit.Divide) and self._fast_div and \
+                isinstance(e[1], myokit.Number):
+            r = self._reciprocal(e[1])
+            return r and (self.ex(e[0]), r)
+        return None
+
+    def _sum(self, e):
+        minus = isinstance(e, myokit.Minus)
+        p = self._product(e[1])
+        if p is not None:
+            a = f'-({p[0]})' if minus else p[0]
+            return self.fma(a, p[1], self.ex(e[0]))
+        p = self._product(e[0])
+        if p is not None:
+            c = self.ex(e[1])
+            return self.fma(p[0], p[1], f'-({c})' if minus else c)
+        return f'({self.ex(e[0])} {"-" if minus else "+"} {self.ex(e[1])})'
+
+    def _scaled_exp(self, x):
+        """
+        exp(k X), k the literal factors of the argument, as
+        2^(X (k log2 e)): mkg_exp_scaled takes the factor in two parts.
+        """
+        k = 1.0
+        while True:
+            if isinstance(x, myokit.PrefixMinus):
+                k, x = -k, x[0]
+            elif isinstance(x, myokit.Multiply) and any(
+                    isinstance(y, myokit.Number) for y in x):
+                i = 0 if isinstance(x[0], myokit.Number) else 1
+                k, x = k * float(x[i].eval()), x[1 - i]
+            elif isinstance(x, myokit.Divide) and isinstance(
+                    x[1], myokit.Number) and float(x[1].eval()) != 0:
+                k, x = k / float(x[1].eval()), x[0]
+            else:
+                break
+        return self.scaled_exp(self.ex(x), k)
+
+    def scaled_exp(self, x, k):
+        """exp(k x) for text x, in single precision."""
+        if not 1e-25 < abs(k) < 1e25:
+            # (outside what two single precision numbers hold)
+            return f'expf(({x}) * {_fmt_number(k, True)})'
+        k *= float(np.log2(np.e))
+        # The next number towards zero: a rest of the same sign, not zero
+        hi = np.float32(k)
+        if abs(float(hi)) >= abs(k):
+            hi = np.nextafter(hi, np.float32(0))
+        return (f'mkg_exp_scaled({x}, {_fmt_number(float(hi), True)}, '
+                f'{_fmt_number(k - float(hi), True)})')
 
     def divide(self, a, b):
         """The quotient of two expressions given as text."""
@@ -138,11 +222,17 @@ class CudaExpressionWriter(CBasedExpressionWriter):
         # quotient), any other one uses the 2-ulp hardware reciprocal.
         num = self.ex(e[0])
         if isinstance(e[1], myokit.Number):
-            d = float(e[1].eval())
-            if d != 0 and np.isfinite(d):
-                r = _fmt_number(float(np.float32(1.0) / np.float32(d)), True)
+            r = self._reciprocal(e[1])
+            if r is not None:
                 return f'(({num}) * {r})'
         return f'__fdividef({num}, {self.ex(e[1])})'
+
+    def _reciprocal(self, e):
+        """The rounded reciprocal of a literal, or None."""
+        d = float(e.eval())
+        if d != 0 and np.isfinite(d):
+            return _fmt_number(float(np.float32(1.0) / np.float32(d)), True)
+        return None
 
     def _fn(self, name):
         if not self._single:
@@ -298,11 +388,30 @@ static __device__ __forceinline__ Real mkg_cubic_root(Real x, Real b, Real c,
 {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        const Real f = ((x + b) * x + c) * x + d;
-        const Real g = (3 * x + 2 * b) * x + c;
+        const Real f = fmaf(fmaf(x + b, x, c), x, d);
+        const Real g = fmaf(fmaf(2, b, 3 * x), x, c);
         if (g != 0) x = x - f / g;
     }
     return x;
+}'''
+
+
+_EXP_HELPER = '''
+// e^(k x), k log2(e) = hi + lo with lo of hi's sign (so that an infinite x
+// gives an infinite exponent): 2^t, t = x (hi + lo) rounded once. Three
+// instructions where the scaled argument and expf take nine, and more
+// exact: neither the rounding of k nor that of the product x k, which grow
+// with the exponent, come in. Root mean square errors on GB300, expf of the
+// product against this: 3.9e-8 and 4.0e-8 for exponents near 0.2, 6.1e-8
+// and 6.2e-8 near 1.3, 1.7e-7 and 1.3e-7 near 5, 6.1e-7 and 3.9e-7 near 16;
+// largest errors 1.42e-7 and 1.37e-7, 2.6e-7 and 2.2e-7, 6.6e-7 and 4.7e-7,
+// 2.3e-6 and 1.4e-6.
+static __device__ __forceinline__ Real mkg_exp_scaled(Real x, Real hi,
+                                                      Real lo)
+{
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaf(x, hi, x * lo)));
+    return r;
 }'''
 
 
@@ -380,7 +489,7 @@ def _pow_helpers(single):
     sq = 'sqrtf' if single else 'sqrt'
     out.append('static __device__ __forceinline__ Real mkg_pow1p5(Real x)'
                f' {{ return x * {sq}(x); }}')
-    out.append(_CUBIC_HELPER if single else _math64())
+    out.extend([_EXP_HELPER, _CUBIC_HELPER] if single else [_math64()])
     return '\n'.join(out)
 
 
@@ -649,7 +758,7 @@ class TissueKernel(object):
     def _generate(self):
         m = self.model
         w = CudaExpressionWriter(self.single, self.native_math,
-                                 self.math == 'fast', soft=True)
+                                 self.math == 'fast', soft=True, fuse=True)
         w.set_lhs_function(self._name)
         real = 'float' if self.single else 'double'
         prec = myokit.SINGLE_PRECISION if self.single else \
@@ -756,6 +865,18 @@ class TissueKernel(object):
             x = literal_subst.get(myokit.Name(var))
             return w.ex(x) if x is not None else self._name(var)
 
+        # Time constants that are reciprocals (1 / (alpha + beta)) by name:
+        # the expression under the line
+        rates = {}
+        for group in order.values():
+            for eq in group.equations(const=False):
+                if isinstance(eq.lhs, myokit.Name) and isinstance(
+                        eq.rhs, myokit.Divide) and isinstance(
+                        eq.rhs[0], myokit.Number) and \
+                        float(eq.rhs[0].eval()) == 1:
+                    rates[eq.lhs.var()] = fold(eq.rhs[1])
+        self.rates = rates
+
         # State loads, and the update of each state, emitted as soon as its
         # inputs exist so that derivatives do not stay live to the end.
         # States in self.hi_states live in the accumulation planes (hi):
@@ -803,10 +924,8 @@ class TissueKernel(object):
                     self._name(v) for v in (inf, tau)
                     if myokit.Name(v) not in literal_subst)
                 inf, tau = ref(inf), ref(tau)
-                expf = w._fn('exp')
-                x = f'mkg_div(-dt_, {tau})' if not self.single else \
-                    f'-dt_ / {tau}'
-                upd = f'{inf} - ({inf} - {n}) * {expf}({x})'
+                decay = self.decay(self.rl_states[s][1], tau, rates)
+                upd = w.fma(f'-({inf} - {n})', decay, inf)
                 text = f'{tab}{target} = {upd};'
                 self._upd_expr[i] = (target, upd)
                 self.census.arith += 4
@@ -816,15 +935,16 @@ class TissueKernel(object):
                 need = set([d])
                 self.census.arith += 2
                 if j is None:
-                    text = f'{tab}{target} = {n} + dt_ * {d};'
-                    self._upd_expr[i] = (target, f'{n} + dt_ * {d}')
+                    upd = w.fma('dt_', d, n)
+                    text = f'{tab}{target} = {upd};'
+                    self._upd_expr[i] = (target, upd)
                 elif self.accumulate == 'double':
                     cur = 'V_' if i == self.i_vm else f'X{n}'
                     dst = target if i == self.i_vm else f'{hiD}[{hplane}]'
                     text = f'{tab}{dst} = {cur} + (double)(dt_ * {d});'
                 else:
                     text = (
-                        f'{tab}{{ const Real y_ = dt_ * {d} - C{n};\n'
+                        f'{tab}{{ const Real y_ = {w.fma("dt_", d, "-C" + n)};\n'
                         f'{tab}  const Real s_ = {n} + y_;\n'
                         f'{tab}  {hiR}[{hplane}] = (s_ - {n}) - y_;\n'
                         f'{tab}  {target} = s_; }}')
@@ -1140,7 +1260,7 @@ class TissueKernel(object):
                 return f'{acc} = -({t});' if first else f'{acc} -= {t};'
             cc = w.ex(myokit.Number(c))
             return (f'{acc} = {cc} * ({t});' if first
-                    else f'{acc} += {cc} * ({t});')
+                    else f'{acc} = {w.fma(cc, t, acc)};')
 
         tab = '            '
         out = []
@@ -1236,10 +1356,29 @@ class TissueKernel(object):
                     acc = f'({acc} + {t})'
                 n = self._name(self.states[i])
                 out.append(f'{tab}        {self._upd_expr[i][0]} = '
-                           f'{n} + dt_ * {acc};')
+                           f'{w.fma("dt_", acc, n)};')
             out.append(f'{tab}    }}')
             out.append(f'{tab}}}')
         return '\n'.join(out)
+
+    def decay(self, var, tau, rates):
+        """
+        exp(-dt / tau) of a Rush-Larsen update: ``tau`` the time constant's
+        text, ``var`` its variable. Where that is a reciprocal 1 / s the
+        exponent is -dt s, one division less.
+        """
+        w = self.writer
+        s = rates.get(var)
+        if s is not None:
+            x = f'dt_ * {w.ex(s)}'
+        elif self.single:
+            x = f'dt_ / {tau}' if self.math != 'fast' else \
+                f'__fdividef(dt_, {tau})'
+        else:
+            x = w.divide('dt_', tau)
+        if self.single and not self.native_math:
+            return w.scaled_exp(x, -1.0)
+        return f'{w._fn("exp")}(-({x}))'
 
     def rhs_code(self, lhs, rhs):
         """CUDA expression for an equation's right-hand side, with the
@@ -1270,7 +1409,8 @@ class TissueKernel(object):
             opts.append('--prec-sqrt=false' if self.native_math else
                         '--prec-sqrt=true')
             opts.append('--ftz=true' if self.math == 'fast' else '--ftz=false')
-        opts.append('--fmad=true')
+        # Multiply-adds are written out (CudaExpressionWriter.ex)
+        opts.append('--fmad=false')
         return opts
 
     def key(self):
