@@ -96,6 +96,12 @@ typedef struct mkg_config {
                                among that many warps, of one CTA or, when
                                more than the CTA holds, of a cluster of
                                whole CTAs (at most 8; 0 is taken as 1) */
+    int32_t team;           /* 0, or warps per tile (1, 2, 4, 8 or 16) of a
+                               resident kernel: every warp tile is a CTA of
+                               32 x team threads that keeps its states in
+                               shared memory for a whole launch, so all of
+                               them must be resident on the device at once;
+                               split and stage are 0 */
 } mkg_config;
 
 /*

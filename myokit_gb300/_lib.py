@@ -54,6 +54,7 @@ class MkgConfig(ctypes.Structure):
         ('stage', ctypes.c_int32),
         ('v_double', ctypes.c_int32),
         ('split', ctypes.c_int32),
+        ('team', ctypes.c_int32),
     ]
 
 

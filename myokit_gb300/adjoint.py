@@ -465,9 +465,15 @@ class TissueAdjoint(object):
                 accumulate=kernel.accumulate,
                 accumulate_states=sim.accumulated_states(), traj=True,
                 stage=kernel.stage, row_pad=kernel.row_pad,
-                stage_lazy=kernel.stage_lazy, sync=kernel.sync)
-            ak = AdjointKernel(fwd, self.min_blocks, self.threads,
-                               self.guards)
+                stage_lazy=kernel.stage_lazy, sync=kernel.sync,
+                team=kernel.team)
+            threads = self.threads
+            if threads is None and kernel.team:
+                # A resident kernel's CTA is one tile; the reverse kernel's
+                # warps each own tiles: as many warps as there are tiles for
+                # an SM
+                threads = 32 * min(kernel.min_blocks, 8)
+            ak = AdjointKernel(fwd, self.min_blocks, threads, self.guards)
             self._generated = {akey: ak}
         key = (id(be), akey, self.segment_steps)
         if self._attached != key:

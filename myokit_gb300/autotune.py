@@ -95,14 +95,43 @@ def lookup(sim):
     return None
 
 
+def resident_shape(tiles, sms, single):
+    """
+    ``(warps per tile, CTAs per SM)`` of a resident kernel
+    (``csrc/resident_kernel.cu.in``) for a grid of ``tiles`` warp tiles, or
+    None where the tiles do not fit on ``sms`` SMs at once.
+
+    The more warps share a tile the shorter is its own step, and the more
+    code an SM has to fetch. Measured, us per step with 1 / 2 / 4 / 8 warps
+    per tile and (last) the undivided kernel, by tiles on an SM:
+
+    - 48 states, single precision: one tile 3.3 / 2.7 / 2.4 / 2.7, 5.3;
+      four 3.3 / 2.7 / 2.5 / 3.3, 5.3; six 3.6 / 2.9 / 3.2, 5.4; eight
+      3.7 / 3.5 / 4.6, 5.5; twelve 4.4 / 5.8, 7.1; sixteen 5.8 / 8.4, 7.4;
+    - the same in double precision: one tile - / - / 25 / 20, 94; two
+      90 / 42 / 29 / -, 93; four 93 / 52 / 47, 95; eight 99 / -, 107;
+    - 8 states, single precision: one 1.21 / 1.11 / 1.08 / 1.15, 2.3; eight
+      1.32 / 1.30 / 1.48, 2.4; sixteen 1.5 / 5.5, 3.1; double precision: one
+      11.9 / 7.6 / 6.5 / 6.6, 14.3; four 12.3 / 8.8 / 7.7 / 8.7, 14.5; six
+      18.7 / 11.7 / 12.3, 18.0; eight 15.2 / 15.4 / 16.8, 18.3.
+    """
+    per = -(-tiles // sms)
+    for team, most in ((4, 4), (2, 8), (1, 16)) if single else (
+            (8, 1), (4, 4), (2, 6), (1, 8)):
+        if per <= most:
+            return team, per
+    return None
+
+
 def _apply(sim, block, min_blocks, spl, lazy=False, sync='barrier',
-           split=1):
+           split=1, team=0):
     sim._block = tuple(block)
     sim._min_blocks = int(min_blocks)
     sim._steps_per_launch = int(spl)
     sim._stage_lazy = int(lazy)
     sim._sync = sync
     sim._split = int(split)
+    sim._team = int(team)
     sim._graphs = 1
 
 
@@ -141,6 +170,18 @@ def _candidates(sim):
     return out
 
 
+def _resident_candidates(sim):
+    """The resident shapes to time on ``sim``: that of its size."""
+    two_d = len(sim._dims) == 2 and sim._diffusion_mode() in (1, 2)
+    nx, ny = (sim._nx, sim._ny) if two_d else (sim._ntotal, 1)
+    shape = resident_shape(-(-nx // 32) * ny, _sm_count(sim._device),
+                           sim._precision == myokit.SINGLE_PRECISION)
+    if shape is None:
+        return []
+    team, minb = shape
+    return [((32 * team, 1), minb, 0, False, _N, 1, team)]
+
+
 def autotune(sim, duration=None, candidates=None, store=True,
              verbose=False):
     """
@@ -151,7 +192,7 @@ def autotune(sim, duration=None, candidates=None, store=True,
     cell-steps per second of device time.
     """
     if candidates is None:
-        candidates = _candidates(sim)
+        candidates = _candidates(sim) + _resident_candidates(sim)
     if duration is None:
         steps = max(20, int(4e8 / sim._ntotal))
         if sim._precision == myokit.DOUBLE_PRECISION:
@@ -159,7 +200,7 @@ def autotune(sim, duration=None, candidates=None, store=True,
         duration = steps * sim.step_size()
     saved = (sim._state.copy(), sim._time, sim._block, sim._min_blocks,
              sim._steps_per_launch, sim._graphs, sim._stage_lazy, sim._sync,
-             sim._split)
+             sim._split, sim._team)
     results = {}
     try:
         for cand in candidates:
@@ -186,7 +227,7 @@ def autotune(sim, duration=None, candidates=None, store=True,
         sim._block, sim._min_blocks = saved[2], saved[3]
         sim._steps_per_launch, sim._graphs = saved[4], saved[5]
         sim._stage_lazy, sim._sync = saved[6], saved[7]
-        sim._split = saved[8]
+        sim._split, sim._team = saved[8], saved[9]
     if not results:
         return None, results
     best = max(results, key=results.get)
@@ -201,6 +242,7 @@ def autotune(sim, duration=None, candidates=None, store=True,
             'stage_lazy': int(best[3]) if len(best) > 3 else 0,
             'sync': best[4] if len(best) > 4 else 'barrier',
             'split': best[5] if len(best) > 5 else 1,
+            'team': best[6] if len(best) > 6 else 0,
             'rate': results[best],
             'when': time.strftime('%Y-%m-%dT%H:%M:%S')}
         try:

@@ -336,6 +336,7 @@ struct mkg_sim {
     mkg_step *d_steps = nullptr;
     mkg_status *d_status = nullptr;
     unsigned int *d_warp_epoch = nullptr;  /* per-warp step counters */
+    void *d_vtag = nullptr;   /* resident kernels: V words with their steps */
     size_t n_warp_epoch = 0;
     double *d_stage = nullptr;   /* staging for double uploads */
     void *d_hi = nullptr;        /* accumulation planes [n_hi][pitch] x 8 B */
@@ -659,6 +660,7 @@ void fill_launch(mkg_sim *s, mkg_launch *a)
     a->wait_skew = s->wait_skew;
     a->hi = s->d_hi;
     a->warp_epoch = s->d_warp_epoch;
+    a->vtag = s->d_vtag;
     /* Warp tiles: 32 consecutive cells of a row (2D) or of the flat cell
      * array (1D cables, connection graphs, diffusion-free simulations). */
     if (s->cfg.two_d) {
@@ -771,7 +773,20 @@ long long blocks_needed(const mkg_sim *s, const mkg_launch *a)
     const long long nwt = (long long)a->ntiles_x * a->ntiles_y;
     const int threads = s->cfg.block_x * s->cfg.block_y;
     const long long split = s->cfg.split > 1 ? s->cfg.split : 1;
+    if (s->cfg.team > 0) return nwt;
     return (nwt * 32 * split + threads - 1) / threads;
+}
+
+/* Step counters and V words start at zero: before the launches of a chunk,
+ * which count its steps from one */
+int reset_step_words(mkg_sim *s)
+{
+    CK(s, cudaMemsetAsync(s->d_warp_epoch, 0,
+                          s->n_warp_epoch * sizeof(unsigned int), s->stream));
+    if (s->d_vtag)
+        CK(s, cudaMemsetAsync(s->d_vtag, 0, (size_t)s->pitch * 2 * 16,
+                              s->stream));
+    return MKG_OK;
 }
 
 }  // namespace
@@ -873,6 +888,7 @@ void mkg_destroy(mkg_sim *s)
     dfree(s->d_steps);
     dfree(s->d_status);
     dfree(s->d_warp_epoch);
+    dfree(s->d_vtag);
     dfree(s->d_stage);
     dfree(s->d_hi);
     dfree(s->d_hi_slot);
@@ -942,6 +958,12 @@ int mkg_create(const mkg_config *cfg, const void *cubin, size_t cubin_size,
                            " per CTA, or teams of 2 to 8 whole CTAs, no"
                            " staging and no accumulation planes");
     }
+    if (cfg->team < 0 || cfg->team > 16 || (cfg->team & (cfg->team - 1)) ||
+        (cfg->team > 0 && (cfg->block_x != 32 * cfg->team || cfg->stage ||
+                           cfg->split > 1)))
+        return set_err(nullptr, MKG_ERR_ARG,
+                       "a resident tile is a CTA of 1, 2, 4, 8 or 16 warps,"
+                       " not staged and not split");
     if (cfg->stage) {
         /* Tensor copy limits: 256 planes per box, int32 coordinates */
         StageLayout L;
@@ -1019,6 +1041,8 @@ int mkg_create(const mkg_config *cfg, const void *cubin, size_t cubin_size,
     }
     CKC(cudaMalloc((void **)&s->d_status, sizeof(mkg_status)));
     CKC(cudaMallocHost((void **)&s->h_status, sizeof(mkg_status)));
+    if (cfg->team > 0 && cfg->diffusion != MKG_DIFF_NONE)
+        CKC(cudaMalloc(&s->d_vtag, (size_t)s->pitch * 2 * 16));
     /* One step counter per warp of the largest co-resident grid */
     s->n_warp_epoch = (size_t)s->occ_blocks * s->num_sms *
                       (size_t)(cfg->block_x / 32);
@@ -1467,6 +1491,12 @@ int mkg_run_chunk(mkg_sim *s, int64_t max_steps, double *t_out,
                                     : s->occ_blocks;
     long long coop_blocks = std::min<long long>(nblocks,
                                                 (long long)bpsm * s->num_sms);
+    if (s->cfg.team > 0 && coop_blocks < nblocks) {
+        s->running = false;
+        return set_err(s, MKG_ERR_ARG,
+                       "a resident kernel needs all %lld tiles on the device"
+                       " at once; %lld fit", nblocks, coop_blocks);
+    }
     /* Split teams larger than the CTA are clusters of whole CTAs */
     const int ncl = cluster_ctas(s);
     coop_blocks -= coop_blocks % ncl;
@@ -1484,8 +1514,8 @@ int mkg_run_chunk(mkg_sim *s, int64_t max_steps, double *t_out,
     *s->h_status = init;
     CK(s, cudaMemcpyAsync(s->d_status, s->h_status, sizeof(mkg_status),
                           cudaMemcpyHostToDevice, s->stream));
-    CK(s, cudaMemsetAsync(s->d_warp_epoch, 0,
-                          s->n_warp_epoch * sizeof(unsigned int), s->stream));
+    r = reset_step_words(s);
+    if (r) return r;
     CK(s, cudaEventRecord(s->ev0, s->stream));
 
     const int64_t nlaunch = (n + spl - 1) / spl;
@@ -2205,10 +2235,9 @@ int adj_backward(mkg_sim *s, const double *lgrad, int64_t rows,
         if (s->cfg.stage) a.stage_tx = (int)s->lay.tx;
         CK(s, cudaMemsetAsync(&s->d_status->barrier, 0, sizeof(unsigned),
                               s->stream));
-        CK(s, cudaMemsetAsync(s->d_warp_epoch, 0,
-                              s->n_warp_epoch * sizeof(unsigned int),
-                              s->stream));
-        int r = launch_coop(s, s->adj_fwd, &a, s->adj_occ_fwd,
+        int r = reset_step_words(s);
+        if (r) return r;
+        r = launch_coop(s, s->adj_fwd, &a, s->adj_occ_fwd,
                             blocks_needed(s, &a), s->tile_smem);
         if (r) return r;
         /* The segment in reverse */

@@ -87,6 +87,9 @@ typedef struct mkg_launch {
                                 of every step, Real[nsteps][n_state][pitch] */
     unsigned int *warp_epoch; /* neighbour synchronisation: steps completed
                                 by each warp of the grid (reset per chunk) */
+    void *vtag;              /* resident kernels: V with the step it belongs
+                                to, [2][pitch] words of 8 (FP32) or 16
+                                bytes, tags reset per chunk */
 } mkg_launch;
 
 /* An opaque TMA tensor map (CUtensorMap: 128 bytes, 64-byte aligned) */

@@ -30,6 +30,13 @@ typedef unsigned long long mkg_u64;
 #ifdef __CUDACC__
 #define MKG_M64 static __device__ __forceinline__
 #define MKG_M64_SLOW static __device__ __noinline__
+/* exp and division proper: inlined, or (MKG_M64_OUTLINE) called, where the
+ * code of a large model would otherwise not fit the instruction caches */
+#ifdef MKG_M64_OUTLINE
+#define MKG_M64_FN MKG_M64_SLOW
+#else
+#define MKG_M64_FN MKG_M64
+#endif
 MKG_M64 mkg_u32 mkg_mulhi(mkg_u32 a, mkg_u32 b) { return __umulhi(a, b); }
 /* Bits 32.. of (hi:lo) << s and bits 0..31 of (hi:lo) >> s, s in 0..31 */
 MKG_M64 mkg_u32 mkg_shl(mkg_u32 lo, mkg_u32 hi, mkg_u32 s)
@@ -79,7 +86,7 @@ MKG_M64 mkg_u64 mkg_mulhi64(mkg_u64 a, mkg_u64 b)
  *   r = j/256 + g: e^r = e^(j/256) (1 + g (1 + g S(g))), S from the series;
  *   rounded to 53 bits, exponent added.
  */
-MKG_M64 double mkg_exp(double x)
+MKG_M64_FN double mkg_exp(double x)
 {
     const mkg_u32 hx = mkg_hi(x), lx = mkg_lo(x);
     const mkg_u32 ax = hx & 0x7fffffffu;
@@ -175,7 +182,7 @@ MKG_M64 double mkg_div_by(double a, double b, mkg_u32 y)
                     (mkg_u32)out);
 }
 
-MKG_M64 double mkg_div(double a, double b)
+MKG_M64_FN double mkg_div(double a, double b)
 {
     /* Leading 32 bits of b's significand (1.31); the reciprocal of its
      * leading 24 bits, rounded up, to an ulp; then one Newton step, taken

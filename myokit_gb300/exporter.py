@@ -35,6 +35,7 @@ import numpy as np
 
 from ._deps import myokit
 from myokit.formats.ansic import CBasedExpressionWriter
+from . import teams as _teams
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_HERE, 'csrc')
@@ -211,6 +212,12 @@ class CudaExpressionWriter(CBasedExpressionWriter):
         if self._soft:
             num, den = self.ex(e[0]), e[1]
             if isinstance(den, myokit.Number):
+                d = float(den.eval())
+                if abs(np.frexp(d)[0]) == 0.5 and 2.0 ** -900 < abs(d) < \
+                        2.0 ** 900:
+                    # A power of two: its reciprocal is exact
+                    return num if d == 1 else \
+                        f'({num} * {_fmt_number(1 / d, False)})'
                 y = _reciprocal_digits(float(den.eval()))
                 if y is not None:
                     return f'mkg_div_by({num}, {self.ex(den)}, {y}u)'
@@ -465,7 +472,7 @@ def cubic_root_coefficients(rhs):
     return None
 
 
-def _pow_helpers(single):
+def _pow_helpers(single, outline=False):
     """Inline helpers for x^n (n = 2..16, by repeated squaring) and x^1.5
     and, in single precision, the cubic root refinement."""
     out = []
@@ -489,6 +496,8 @@ def _pow_helpers(single):
     sq = 'sqrtf' if single else 'sqrt'
     out.append('static __device__ __forceinline__ Real mkg_pow1p5(Real x)'
                f' {{ return x * {sq}(x); }}')
+    if not single and outline:
+        out.append('#define MKG_M64_OUTLINE')
     out.extend([_EXP_HELPER, _CUBIC_HELPER] if single else [_math64()])
     return '\n'.join(out)
 
@@ -629,7 +638,7 @@ class TissueKernel(object):
                  fast_divide=True, min_blocks=1, math='default',
                  accumulate=None, accumulate_states=(), traj=False,
                  stage=False, row_pad=False, stage_lazy=False,
-                 sync='barrier', split=1):
+                 sync='barrier', split=1, team=0):
         self.model = model
         self.single = (precision == myokit.SINGLE_PRECISION)
         self.native_math = bool(native_math)
@@ -696,6 +705,18 @@ class TissueKernel(object):
         if self.split > 1:
             stage = False
             sync = 'barrier'
+        asked = bool(stage)
+        # Warps per tile of a resident kernel (0: not resident): the tile is
+        # a CTA, keeps its states in shared memory for a whole launch and
+        # exchanges V with its neighbours word by word
+        self.team = int(team)
+        if self.team not in (0, 1, 2, 4, 8, 16):
+            raise ValueError('team must be 0, 1, 2, 4, 8 or 16')
+        if self.team:
+            if self.block != (32 * self.team, 1) or self.split > 1:
+                raise ValueError('a resident tile is a CTA of its own')
+            stage = False
+            sync = 'neighbors'
         self.stage = bool(stage)
         self.row_pad = bool(row_pad) and self.two_d
         self.stage_lazy = int(stage_lazy)
@@ -725,6 +746,7 @@ class TissueKernel(object):
                 # Two buffers per warp only where they fit
                 if self.stage_lazy == 2 and 2 * per_cta > STAGE_MAX_CTA:
                     self.stage_lazy = 1
+        self.team_nslot = 0
         # Staging buffers per warp (mkg_config.stage)
         self.stage_buffers = 2 if self.layout and self.stage_lazy == 2 \
             else 1
@@ -733,6 +755,9 @@ class TissueKernel(object):
         # formula, refined by mkg_cubic_root: name -> (b, c, d) names
         self.cubic = {}
         self._source = self._generate()
+        if self.team and asked:
+            # The resident tile's shared memory, where staging was asked for
+            self.layout = {'bytes': self.resident_bytes()}
 
     # -- naming ------------------------------------------------------------
 
@@ -845,9 +870,14 @@ class TissueKernel(object):
 
         def item(lhs, rhs, line):
             refs = set(self._name(r) for r in rhs.references())
-            c = OpCensus()
-            c.add(rhs)
-            items.append((self._name(lhs), refs, line, c.cost()))
+            if self.team:
+                c = _teams.cost(rhs, self.single) + (
+                    30 if self._name(lhs) in self.cubic else 0)
+            else:
+                c = OpCensus()
+                c.add(rhs)
+                c = c.cost()
+            items.append((self._name(lhs), refs, line, c))
 
         body.append(tab + '// Per-cell constants (scalar fields)')
         for eq in const_eqs:
@@ -1018,7 +1048,7 @@ class TissueKernel(object):
         log_a = _LOG_BLOCK.format(
             cond=f'item <= {self.n_state}',
             cases=('\n' + t2 + '        ').join(cases))
-        if self.traj:
+        if self.traj and not self.team:
             # The adjoint's forward pass records the states at t of every
             # step of the launch: traj[k][state][pitch]. Written with the
             # logged values, so by the lanes that hold a cell only: staged
@@ -1040,6 +1070,8 @@ class TissueKernel(object):
                 cond=f'item > {self.n_state}',
                 cases=('\n' + t2 + '        ').join(cases))
 
+        if self.team:
+            return self._resident(items, log_a, log_b)
         split_body = ''
         if self.split > 1:
             split_body = self._split_body(
@@ -1047,6 +1079,7 @@ class TissueKernel(object):
         self.split_body = split_body
 
         subs = {
+            '@DEVICE@': _read('mkg_device.h'),
             '@SPLIT@': str(self.split),
             '@SPLIT_CL@': str(self.split_cl),
             '@SPLIT_NSLOT@': str(self.split_nslot),
@@ -1106,6 +1139,253 @@ class TissueKernel(object):
         return (
             '// Generated by myokit_gb300.exporter for model '
             + str(m.name()) + '\n' + abi + '\n' + text)
+
+    def host_stage(self):
+        """Staging buffers per warp as the host has to lay them out."""
+        return self.stage_buffers if self.layout and not self.team else 0
+
+    # -- resident kernels ----------------------------------------------------
+
+    def resident_bytes(self):
+        """Static shared memory of a resident tile."""
+        r = 4 if self.single else 8
+        n = self.n_state + len(self.fields) + self.team_nslot
+        hi = {None: 0, 'double': 8, 'kahan': 4}[self.accumulate]
+        return 32 * (n * r + len(self.hi_states) * hi +
+                     (8 if self.v_double else r)) + 16
+
+    def _resident(self, items, log_a, log_b):
+        """Source of the resident kernel (csrc/resident_kernel.cu.in)."""
+        w = self.writer
+        real = 'float' if self.single else 'double'
+        tab = '            '
+        index = {self._name(s): i for i, s in enumerate(self.states)}
+        line_of = {name: line for name, _, line, _ in items}
+        refs = {name: r for name, r, _, _ in items}
+        rate_refs = {v: set(self._name(r) for r in e.references())
+                     for v, e in self.rates.items()}
+        gates, derivatives = {}, {}
+        for i, s in enumerate(self.states):
+            if s in self.rl_states:
+                inf, tau = self.rl_states[s]
+                gates[i] = set(self._name(v) for v in (inf, tau)
+                               if myokit.Name(v) not in self.literal_subst)
+                if tau in self.rates:
+                    # (the sum under the line stands in its place)
+                    gates[i].discard(self._name(tau))
+                    gates[i] |= rate_refs[tau]
+                gates[i] &= set(refs)
+            else:
+                derivatives[i] = self._name(s.lhs())
+        # (in evaluation order: what a phase refers to is defined before)
+        first = self.i_vm if self.i_vm in derivatives else None
+        team = _teams.Team(
+            self.team, [(n, r, c) for n, r, _, c in items], gates,
+            derivatives, first, _IDIFF,
+            _teams._COST[self.single]['rl'])
+        self.team_plan = team
+        self.team_nslot = len(team.slots)
+        halo = [p for p in range(self.team) if team.halo[p] or p == 0] \
+            if self.diffusion != DIFF_NONE else []
+        hi = self.accumulate
+
+        def loads(names):
+            out = []
+            for n in sorted(names & set(index), key=index.get):
+                i = index[n]
+                if i == self.i_vm:
+                    out.append(f'{tab}    const Real {n} = (Real)vs[lane];')
+                else:
+                    out.append(f'{tab}    const Real {n} = xs[{i}][lane];')
+            for k, v in enumerate(self.fields):
+                if self._name(v) in names:
+                    out.append(f'{tab}    const Real {self._name(v)} = '
+                               f'fs[{k}][lane];')
+            return out
+
+        def update(i):
+            """(statements before the team meets, after) of a state."""
+            s = self.states[i]
+            n = self._name(s)
+            j = self.hi_index.get(i)
+            if i in gates:
+                a = [f'const Real n{i}_ = {self._upd_expr[i][1]};']
+                new = f'n{i}_'
+                b = []
+            elif j is None:
+                a, b = [], [f'const Real n{i}_ = {self._upd_expr[i][1]};']
+                new = f'n{i}_'
+            elif hi == 'double':
+                d = derivatives[i]
+                cur = 'vs[lane]' if i == self.i_vm else f'xd[{j}][lane]'
+                a = []
+                b = [f'const double n{i}_ = {cur} + (double)(dt_ * {d});']
+                if i != self.i_vm:
+                    b.append(f'xd[{j}][lane] = n{i}_;')
+                new = f'n{i}_' if i == self.i_vm else f'(Real)n{i}_'
+            else:
+                d = derivatives[i]
+                y = w.fma('dt_', d, f'-xc[{j}][lane]')
+                a = []
+                b = [f'const Real y{i}_ = {y};',
+                     f'const Real n{i}_ = {n} + y{i}_;',
+                     f'xc[{j}][lane] = (n{i}_ - {n}) - y{i}_;']
+                new = f'n{i}_'
+            if i == self.i_vm:
+                b.append(f'vs[lane] = {new};')
+                b.append('if (k + 1 < nsteps && live)\n' + tab +
+                         f'        mkg_word_store(vout_, cid, {new},'
+                         ' now_ + 1u);')
+            else:
+                b.append(f'xs[{i}][lane] = {new};')
+            return a, b
+
+        # Logged values at t: the states from their columns, logged
+        # intermediaries computed again (the first warp, at log rows only)
+        log = log_a
+        for n, i in index.items():
+            col = '(Real)vs[lane]' if i == self.i_vm else f'xs[{i}][lane]'
+            log = log.replace(f'val = {n};', f'val = {col};')
+        n0 = self._name(self.states[0])
+        col0 = '(Real)vs[lane]' if self.i_vm == 0 else 'xs[0][lane]'
+        log = log.replace(f'isnan({n0})', f'isnan({col0})')
+        inter = []
+        if self.inter_log:
+            todo = list(self._inter_names)
+            names = set()
+            while todo:
+                x = todo.pop()
+                if x in names or x not in refs:
+                    continue
+                names.add(x)
+                todo.extend(refs[x])
+            used = set(self._inter_names).union(*[refs[x] for x in names]) \
+                if names else set(self._inter_names)
+            inter = [f'{tab}    {{'] + loads(used) + [
+                line_of[n] for n, _, _, _ in items if n in names] + [
+                f'{tab}    if (live) {{', log_b, f'{tab}    }}',
+                f'{tab}    }}']
+
+        out = []
+        nphase = len(team.work)
+        for p in range(self.team):
+            gate_list = [i for f in range(nphase) for i in team.gates_of[f][p]]
+            names = set()
+            for f in range(nphase):
+                for x in team.work[f][p]:
+                    names |= refs[x]
+            for i in gate_list + team.tails_of[p]:
+                names.add(self._name(self.states[i]))
+                if i in gates:
+                    inf, tau = self.rl_states[self.states[i]]
+                    names |= gates[i] | rate_refs.get(tau, set())
+                    names.add(self._name(inf))
+            out.append(f'{tab}{"if" if p == 0 else "else if"} (part_ == {p})'
+                       ' {')
+            out.extend(loads(names))
+            take = [f'{tab}    MKG_HALO(id_)',
+                    f'{tab}    const Real {_IDIFF} = (Real)id_;',
+                    f'{tab}    (void){_IDIFF};']
+            if not halo:
+                take = [f'{tab}    const Real {_IDIFF} = 0;',
+                        f'{tab}    (void){_IDIFF};']
+            early = p in halo and team.halo_early[p]
+            if early:
+                out.extend(take)
+            if p == 0:
+                # Logged values, before any state changes; a NaN halt
+                out.append(f'{tab}    if (row >= 0) {{')
+                if not early:
+                    out.extend(take)
+                out.append(f'{tab}    if (live) {{')
+                out.append(log)
+                out.append(f'{tab}    }}')
+                out.extend(inter)
+                out.append(f'{tab}    }}')
+                out.append(f'{tab}    MKG_CHECK_HALT()')
+            after = []           # stores that wait for the team's loads
+            for f in range(nphase):
+                if f:
+                    out.append(f'{tab}    mkg_team_sync();')
+                if f == 1:
+                    out.append(f'{tab}    if (s_stop) break;')
+                    out.extend(after)
+                    after = []
+                for x in team.read[f][p]:
+                    out.append(f'{tab}    const Real {x} = '
+                               f'hs[{team.slots[x]}][lane];')
+                if f == nphase - 1 and (p in halo or (p == 0 and not halo)) \
+                        and not early and (team.halo[p] or p == 0):
+                    out.extend(take)
+                out.extend(line_of[x] for x in team.work[f][p])
+                for x in team.written[f][p]:
+                    out.append(f'{tab}    hs[{team.slots[x]}][lane] = {x};')
+                for i in team.gates_of[f][p]:
+                    a, b = update(i)
+                    out.extend(f'{tab}    {x}' for x in a)
+                    (out if f else after).extend(f'{tab}    {x}' for x in b)
+            if nphase == 1:
+                # (a team of one warp: nothing changes hands)
+                out.append(f'{tab}    mkg_team_sync();')
+                out.append(f'{tab}    if (s_stop) break;')
+                out.extend(after)
+            for i in team.tails_of[p]:
+                for x in sum(update(i), []):
+                    out.append(f'{tab}    {x}')
+            if p == 0:
+                out.append(f'{tab}    if (tile == 0 && row >= 0 && '
+                           'a.nan_check && lane == 0 && k + 1 < nsteps)')
+                out.append(f'{tab}        mkg_st_release(a.warp_epoch, '
+                           'now_ + 1u);')
+            out.append(f'{tab}}}')
+        self.team_body = '\n'.join(out)
+        subs = {
+            '@TEAM_BODY@': self.team_body,
+            '@REAL@': real,
+            '@VREAL@': 'double' if self.v_double else real,
+            '@SINGLE@': '1' if self.single else '0',
+            '@V_DOUBLE@': '0' if self.single and not self.v_double else '1',
+            '@N_STATE@': str(self.n_state),
+            '@N_FIELD@': str(len(self.fields)),
+            '@N_HI@': str(len(self.hi_states)),
+            '@HI_MODE@': {None: '0', 'double': '1', 'kahan': '2'}[
+                hi if self.hi_states else None],
+            '@I_VM@': str(self.i_vm),
+            '@DIFF@': str(self.diffusion),
+            '@TWO_D@': '1' if self.two_d else '0',
+            '@TEAM@': str(self.team),
+            '@NSLOT@': str(self.team_nslot),
+            '@TRAJ@': '1' if self.traj else '0',
+            '@TRAJ_VALUE@': 'xs[i][lane]',
+            '@DEVICE@': _read('mkg_device.h'),
+            '@FIELD_LOADS@': '\n'.join(
+                f'        if (part_ == {k % self.team}) fs[{k}][lane] = '
+                f'field[(long long){k} * pitch + cid];'
+                for k in range(len(self.fields))),
+            '@HI_LOADS@': '\n'.join(
+                f'        if (part_ == {i % self.team}) xs[{i}][lane] = '
+                f'(Real)((const double *)a.hi)[(long long){j} * pitch + cid];'
+                for i, j in self.hi_index.items() if i != self.i_vm),
+            '@MINB@': str(self.min_blocks),
+            # A tile's warps run a step's code once each, from the
+            # instruction caches (32 KB an SM, some 128 KB shared by ten SMs
+            # or so). With exp and division (75 and 65 instructions) inlined,
+            # the 48-state model's double precision code is 430 KB: 152 tiles
+            # took 42 us a step, with both called 20 us; 304 tiles 82 and 29
+            # us. A small model's code fits: Beeler-Reuter (2600 instructions
+            # of them) 4.0 us inlined, 4.2 us called.
+            '@POW_HELPERS@': _pow_helpers(
+                self.single, 75 * self.census.trans +
+                65 * self.census.divide > 6000),
+            '@NEED_HALO@': ' || '.join(f'part_ == {p}' for p in halo)
+            or 'false',
+                    }
+        text = _read('resident_kernel.cu.in')
+        for k, v in subs.items():
+            text = text.replace(k, v)
+        return ('// Generated by myokit_gb300.exporter for model '
+                + str(self.model.name()) + '\n' + _read('mkg_kernel_abi.h')
+                + '\n' + text)
 
     def _split_terms(self, rhs_of):
         """

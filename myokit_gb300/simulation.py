@@ -264,6 +264,9 @@ class SimulationCUDA(object):
         self._sync = None
         # Warps per warp tile (1, 2, 4, 8 or 16); None: tuned or 1
         self._split = None
+        # Warps per tile of a resident kernel (0: not resident); None: tuned
+        # or by size (resident_shape)
+        self._team = None
         if accumulate not in (None, 'double', 'kahan'):
             raise ValueError(
                 'The argument "accumulate" must be None, "double" or'
@@ -875,23 +878,59 @@ class SimulationCUDA(object):
                 out.append(st)
         return out
 
+    def _resident(self, two_d):
+        """
+        ``(warps per tile, CTAs per SM)`` of a resident kernel, or None. By
+        size where neither the caller nor a tuner chose a launch shape.
+        """
+        from . import autotune
+        nx, ny = (self._nx, self._ny) if two_d else (self._ntotal, 1)
+        tiles = -(-nx // 32) * ny
+        if self._team is not None:
+            if not self._team:
+                return None
+            return self._team, max(1, self._min_blocks or 1)
+        if not all(x is None for x in (self._block, self._split, self._sync,
+                                       self._stage_lazy, self._min_blocks)):
+            return None
+        hit = self._tuned_choice()
+        if hit is not None:
+            if not hit.get('team'):
+                return None
+            return int(hit['team']), int(hit['min_blocks'])
+        return autotune.resident_shape(
+            tiles, autotune._sm_count(self._device),
+            self._precision == myokit.SINGLE_PRECISION)
+
     def _kernel(self, inter_log):
         """The generated kernel for the current configuration (cached)."""
         mode = self._diffusion_mode()
         two_d = len(self._dims) == 2 and mode in (
             _exp.DIFF_GRID, _exp.DIFF_HETERO)
+        res = self._resident(two_d)
+        if res is not None:
+            k = self._make_kernel(inter_log, mode, two_d, (32 * res[0], 1),
+                                  res[1], res[0])
+            # (a model too large for that many tiles on an SM)
+            if k.resident_bytes() <= 48 * 1024 and \
+                    k.resident_bytes() * res[1] <= 216 * 1024:
+                return k
         block = self._block_shape(two_d)
-        minb = self._default_min_blocks(block)
+        return self._make_kernel(inter_log, mode, two_d, block,
+                                 self._default_min_blocks(block), 0)
+
+    def _make_kernel(self, inter_log, mode, two_d, block, minb, team):
         acc = self.accumulated_states()
         # Tile staging with TMA for grids of at least 256 cells; rows that
         # are not a multiple of 4 cells need the padded copy width
         stage = self._stage_tiles and self._ntotal >= 256
         row_pad = two_d and self._nx % 4 != 0
-        lazy = stage and self._lazy_staging()
-        key = (
+        lazy = 0 if team else stage and self._lazy_staging()
+        split = 1 if team else self._split_mode()
+        key = (team,
             self._model_version, self._precision, self._native_math, mode,
             two_d, block, minb, self._fp32_math, self._accumulate,
-            stage, row_pad, lazy, self._sync_mode(), self._split_mode(),
+            stage, row_pad, lazy, self._sync_mode(), split,
             tuple(v.qname() for v in acc),
             tuple(v.qname() for v in self._fields.keys()),
             tuple(v.qname() for v in inter_log))
@@ -904,7 +943,7 @@ class SimulationCUDA(object):
                 min_blocks=minb, math=self._fp32_math,
                 accumulate=self._accumulate, accumulate_states=acc,
                 stage=stage, row_pad=row_pad, stage_lazy=lazy,
-                sync=self._sync_mode(), split=self._split_mode())
+                sync=self._sync_mode(), split=split, team=team)
             if len(self._kernels) > 16:
                 self._kernels.clear()
             self._kernels[key] = k
@@ -928,7 +967,8 @@ class SimulationCUDA(object):
         cfg.hi_mode = {None: 0, 'double': 1, 'kahan': 2}[kernel.accumulate] \
             if kernel.hi_states else 0
         cfg.n_hi = len(kernel.hi_states)
-        cfg.stage = kernel.stage_buffers if kernel.layout else 0
+        cfg.stage = kernel.host_stage()
+        cfg.team = kernel.team
         cfg.v_double = 1 if kernel.v_double else 0
         cfg.split = kernel.split
         key = (kernel.key(), bytes(cfg))

@@ -27,6 +27,7 @@ typedef unsigned long long mkg_u64;
 @TABLE@
 #define MKG_M64 static inline
 #define MKG_M64_SLOW static inline
+#define MKG_M64_FN static inline
 static int ulp = 0;
 MKG_M64 mkg_u32 mkg_mulhi(mkg_u32 a, mkg_u32 b)
 { return (mkg_u32)(((mkg_u64)a * b) >> 32); }
