@@ -108,19 +108,53 @@ def resident_shape(tiles, sms, single):
     - 48 states, single precision: one tile 3.3 / 2.7 / 2.4 / 2.7, 5.3;
       four 3.3 / 2.7 / 2.5 / 3.3, 5.3; six 3.6 / 2.9 / 3.2, 5.4; eight
       3.7 / 3.5 / 4.6, 5.5; twelve 4.4 / 5.8, 7.1; sixteen 5.8 / 8.4, 7.4;
-    - the same in double precision: one tile - / - / 25 / 20, 94; two
-      90 / 42 / 29 / -, 93; four 93 / 52 / 47, 95; eight 99 / -, 107;
+    - the same in double precision: one tile 71 / 36 / 21 / 15, 93; two
+      71 / 36 / 23 / 28, 93; three - / 39 / 29 / 42, 93; four 73 / 40 / 51,
+      95; six 78 / 56 / 71, 98; seven 78 / 75; eight 80 / 81, 107;
     - 8 states, single precision: one 1.21 / 1.11 / 1.08 / 1.15, 2.3; eight
       1.32 / 1.30 / 1.48, 2.4; sixteen 1.5 / 5.5, 3.1; double precision: one
-      11.9 / 7.6 / 6.5 / 6.6, 14.3; four 12.3 / 8.8 / 7.7 / 8.7, 14.5; six
-      18.7 / 11.7 / 12.3, 18.0; eight 15.2 / 15.4 / 16.8, 18.3.
+      11.9 / 7.6 / 6.5 / 6.6, 14.3; three - / 8.4 / 6.9 / 7.1; six 18.7 /
+      11.7 / 12.3, 18.0; eight 15.2 / 15.4 / 16.8, 18.3.
+
+    Nine tiles on an SM in double precision take 100 us with the 48 states,
+    the undivided kernel 94: its 8 warps per SM have the registers they need.
     """
     per = -(-tiles // sms)
     for team, most in ((4, 4), (2, 8), (1, 16)) if single else (
-            (8, 1), (4, 4), (2, 6), (1, 8)):
+            (8, 1), (4, 3), (2, 7), (1, 8)):
         if per <= most:
             return team, per
     return None
+
+
+def default_shape(single, n_state, plane_bytes):
+    """
+    The launch shape of a grid too large for resident tiles, where nobody
+    chose one: ``(threads, CTAs per SM, lazy staging, synchronisation)``.
+    ``plane_bytes``: the states and accumulation planes of all cells.
+
+    Measured, us per step:
+
+    - single precision, planes beyond the L2 (129 MB): 512 threads with
+      neighbour waits, 48 states: 2048 x 2048 Kahan 366 against 417 with 256
+      x 2 and the grid barrier, 1024 x 1024 Kahan 86 and 104, 1531 x 777 86
+      and 101; 8 states 2048 x 2048 74 and 74. The many tiles of a warp
+      even out what neighbours wait for, and no warp idles at a barrier
+      while memory does;
+    - planes within it: 256 x 2 with the barrier (512 x 512, 48 states: 20.7
+      against 20.3, 300 x 400 per-edge 13.1 and 13.4, 8 states 6.3 and 6.9);
+    - double precision, many states: 8 warps per SM of 64-thread CTAs, read
+      from shared memory where used: 256 x 256 114 against 180 with 128
+      threads and prefetch, 301 x 211 119 and 182, 512 x 512 491 and 676;
+    - double precision, few states (registers do not limit the warps): 512
+      threads, 512 x 512 with 8 states 79 against 85; 64-thread CTAs 100.
+    """
+    if not single:
+        return (64, 4, 1, 'barrier') if n_state >= 16 else (
+            512, 1, 1, 'barrier')
+    if plane_bytes > 120e6:
+        return 512, 1, 0, 'neighbors'
+    return 256, 2, 0, 'barrier'
 
 
 def _apply(sim, block, min_blocks, spl, lazy=False, sync='barrier',

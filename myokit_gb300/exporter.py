@@ -67,6 +67,20 @@ def _fmt_number(x, single):
     return s + 'f' if single else s
 
 
+def third_of_acos(e):
+    """z if ``e`` is acos(z) / 3 (as cubic roots have it), or None."""
+    n = myokit.Number
+    if isinstance(e, myokit.Divide) and isinstance(e[0], myokit.ACos) and \
+            isinstance(e[1], n) and float(e[1].eval()) == 3:
+        return e[0][0]
+    if isinstance(e, myokit.Multiply):
+        for a, b in ((e[0], e[1]), (e[1], e[0])):
+            if isinstance(a, myokit.ACos) and isinstance(b, n) and \
+                    float(b.eval()) == 1 / 3:
+                return a[0]
+    return None
+
+
 def _reciprocal_digits(x):
     """
     2^32 / (the significand of a normal ``x``, in [1, 2)), rounded down and
@@ -78,15 +92,26 @@ def _reciprocal_digits(x):
                (1 << 32) - 1)
 
 
-def _exp_table():
-    """The table of mkg_exp: e^(j/256) in units of 2^-62, j = 0 .. 178."""
+def _math_tables():
+    """
+    The tables of mkg_math64.h: e^(j/256) in units of 2^-62, j = 0 .. 178;
+    and by the leading 8 bits of a significand m in [1, 2), -log(c/2048) in
+    units of 2^-64 and c = 2048/m rounded up (at the low end of its range).
+    """
     from decimal import Decimal, localcontext
-    with localcontext() as c:
-        c.prec = 40
-        v = [int((Decimal(j) / 256).exp() * 2**62 + Decimal('0.5'))
+    with localcontext() as ctx:
+        ctx.prec = 40
+        half = Decimal('0.5')
+        e = [int((Decimal(j) / 256).exp() * 2**62 + half)
              for j in range(179)]
-    return ('static __device__ const unsigned long long mkg_exp_tab[179] = {'
-            + ', '.join('0x%xull' % x for x in v) + '};')
+        t = []
+        for j in range(256):
+            c = -(-2048 * 256 // (256 + j))
+            t += [int(-(Decimal(c) / 2048).ln() * 2**64 + half), c]
+    return '\n'.join(
+        'static __device__ const unsigned long long %s[%d] = {%s};' % (
+            name, len(v), ', '.join('0x%xull' % x for x in v))
+        for name, v in (('mkg_exp_tab', e), ('mkg_log_tab', t)))
 
 
 _MATH64 = []
@@ -95,7 +120,7 @@ _MATH64 = []
 def _math64():
     """Text of the integer exp and division of double precision kernels."""
     if not _MATH64:
-        _MATH64.append(_exp_table() + '\n' + _read('mkg_math64.h'))
+        _MATH64.append(_math_tables() + '\n' + _read('mkg_math64.h'))
     return _MATH64[0]
 
 
@@ -243,7 +268,9 @@ class CudaExpressionWriter(CBasedExpressionWriter):
 
     def _fn(self, name):
         if not self._single:
-            return 'mkg_exp' if self._soft and name == 'exp' else name
+            if self._soft and name in ('exp', 'log', 'sqrt'):
+                return 'mkg_' + name
+            return name
         if self._native and name in ('exp', 'log', 'sin', 'cos', 'tan',
                                      'log10'):
             return '__' + name + 'f'
@@ -266,6 +293,10 @@ class CudaExpressionWriter(CBasedExpressionWriter):
             if p == 1.5:
                 b = self.ex(base)
                 return f'mkg_pow1p5({b})'
+            if self._soft and 2.0 ** -8 <= abs(p) < 16:
+                return (f'mkg_pow_literal({self.ex(base)}, '
+                        f'{self.ex(exponent)}, {int(abs(p) * 2 ** 60)}ull, '
+                        f'{"~0u" if p < 0 else "0u"})')
         return f'{self._fn("pow")}({self.ex(base)}, {self.ex(exponent)})'
 
     def _ex_sqrt(self, e):
@@ -275,6 +306,10 @@ class CudaExpressionWriter(CBasedExpressionWriter):
         return self._ex_function(e, self._fn('sin'))
 
     def _ex_cos(self, e):
+        if self._soft:
+            z = third_of_acos(e[0])
+            if z is not None:
+                return f'mkg_cos_third({self.ex(z)})'
         return self._ex_function(e, self._fn('cos'))
 
     def _ex_tan(self, e):
@@ -476,6 +511,10 @@ def _pow_helpers(single, outline=False):
     """Inline helpers for x^n (n = 2..16, by repeated squaring) and x^1.5
     and, in single precision, the cubic root refinement."""
     out = []
+    if not single:
+        if outline:
+            out.append('#define MKG_M64_OUTLINE')
+        out.append(_math64())
     for n in range(2, 17):
         lines = []
         # binary exponentiation, most significant bit first
@@ -493,12 +532,11 @@ def _pow_helpers(single, outline=False):
         out.append(
             f'static __device__ __forceinline__ Real mkg_pow{n}(Real x)\n'
             '{\n' + '\n'.join(lines) + f'\n    return {cur};\n}}')
-    sq = 'sqrtf' if single else 'sqrt'
+    sq = 'sqrtf' if single else 'mkg_sqrt'
     out.append('static __device__ __forceinline__ Real mkg_pow1p5(Real x)'
                f' {{ return x * {sq}(x); }}')
-    if not single and outline:
-        out.append('#define MKG_M64_OUTLINE')
-    out.extend([_EXP_HELPER, _CUBIC_HELPER] if single else [_math64()])
+    if single:
+        out.extend([_EXP_HELPER, _CUBIC_HELPER])
     return '\n'.join(out)
 
 

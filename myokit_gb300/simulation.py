@@ -778,6 +778,22 @@ class SimulationCUDA(object):
             self._tune_hit = autotune.lookup(self)
         return self._tune_hit
 
+    def _default_shape(self):
+        """
+        The launch shape by size (autotune.default_shape), or None where the
+        caller or a tuner chose one.
+        """
+        if self._block is not None or self._min_blocks is not None or \
+                self._tuned_choice() is not None:
+            return None
+        from . import autotune
+        single = self._precision == myokit.SINGLE_PRECISION
+        planes = self._nstate * (4 if single else 8)
+        if self._accumulate:
+            planes += 4 * len(self.accumulated_states())
+        return autotune.default_shape(single, self._nstate,
+                                      planes * self._ntotal)
+
     def _sync_mode(self):
         """How steps are separated: 'barrier' or 'neighbors'."""
         if self._sync is not None:
@@ -786,7 +802,8 @@ class SimulationCUDA(object):
             hit = self._tuned_choice()
             if hit is not None:
                 return hit.get('sync', 'barrier')
-        return 'barrier'
+        shape = self._default_shape()
+        return 'barrier' if shape is None else shape[3]
 
     def _split_mode(self):
         """Warps that share each warp tile's work (1, 2, 4, 8 or 16)."""
@@ -807,15 +824,19 @@ class SimulationCUDA(object):
             hit = self._tuned_choice()
             if hit is not None:
                 return int(hit.get('stage_lazy', 0))
-        return 0
+        shape = self._default_shape()
+        return 0 if shape is None else shape[2]
 
     def _block_shape(self, two_d):
         """CTA shape (threads, 1); threads is a multiple of the warp size."""
         b = self._block
         if b is None:
             hit = self._tuned_choice()
+            shape = self._default_shape()
             if hit is not None:
                 b = tuple(hit['block'])
+            elif shape is not None:
+                b = shape[0]
             elif self._precision == myokit.DOUBLE_PRECISION:
                 b = 128
             else:
@@ -834,6 +855,9 @@ class SimulationCUDA(object):
             hit = self._tuned_choice()
             if hit is not None:
                 return int(hit['min_blocks'])
+        shape = self._default_shape()
+        if shape is not None:
+            return shape[1]
         if self._precision == myokit.DOUBLE_PRECISION:
             return 1
         # 128 registers per thread: 64K registers / 512 threads

@@ -24,7 +24,7 @@ from ._deps import myokit
 _COST = {
     True: {'div': 5, 'exp': 5, 'log': 16, 'sqrt': 11, 'trig': 20, 'pow': 25,
            'cond': 1, 'rl': 10},
-    False: {'div': 4, 'exp': 6, 'log': 33, 'sqrt': 10, 'trig': 22, 'pow': 98,
+    False: {'div': 4, 'exp': 6, 'log': 7, 'sqrt': 5, 'trig': 22, 'pow': 14,
             'cond': 1, 'rl': 9},
 }
 # Intermediate variables this cheap are evaluated where they are used
@@ -38,6 +38,7 @@ _HALO = 40
 
 def cost(e, single):
     """Estimated time of an expression (see above)."""
+    from . import exporter as _exp
     c = _COST[single]
     t = 0
     for x in e.walk():
@@ -55,6 +56,10 @@ def cost(e, single):
             t += c['log']
         elif isinstance(x, myokit.Sqrt):
             t += c['sqrt']
+        elif isinstance(x, myokit.Cos) and not single and \
+                _exp.third_of_acos(x[0]) is not None:
+            # (one root of a cubic instead of both functions)
+            t += 10 - c['trig'] - c['div']
         elif isinstance(x, (myokit.Sin, myokit.Cos, myokit.Tan, myokit.ASin,
                             myokit.ACos, myokit.ATan)):
             t += c['trig']

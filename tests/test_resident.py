@@ -110,6 +110,28 @@ def test_shape_by_size():
         assert shape(152 * most + 1, 152, single) is None
 
 
+def test_launch_shape_of_large_grids(decker, br77):
+    for m, rl, precision, n, kw, want in (
+            (decker, True, SP, (512, 512), {}, (256, 2, 0, 'barrier')),
+            (decker, True, SP, (1024, 1024), {}, (512, 1, 0, 'neighbors')),
+            (decker, True, SP, (800, 790), {'accumulate': 'kahan'},
+             (512, 1, 0, 'neighbors')),
+            (decker, True, DP, (512, 512), {}, (64, 4, 1, 'barrier')),
+            (br77, False, DP, (512, 512), {}, (512, 1, 1, 'barrier')),
+            (br77, False, SP, (512, 512), {}, (256, 2, 0, 'barrier'))):
+        s = mg.SimulationCUDA(m, None, ncells=n, precision=precision, rl=rl,
+                              **kw)
+        k = s._kernel([])
+        assert (k.block[0], k.min_blocks, k.stage_lazy, k.sync) == want
+        assert k.layout and not k.team
+        # An explicit launch shape is taken as before
+        s = mg.SimulationCUDA(m, None, ncells=n, precision=precision, rl=rl,
+                              block=96, min_blocks=1, **kw)
+        k = s._kernel([])
+        assert (k.block[0], k.min_blocks, k.stage_lazy, k.sync) == (
+            96, 1, 0, 'barrier')
+
+
 def test_large_models_and_launch_options_are_not_resident(br77):
     s = mg.SimulationCUDA(br77, None, ncells=64)
     assert s._kernel([]).team == 4
