@@ -198,6 +198,7 @@ class AdjointKernel(object):
         if self.threads % 32 or not 32 <= self.threads <= 1024:
             raise ValueError('threads must be a multiple of 32 up to 1024')
         self.guards = bool(guards)
+        self._key = None
         self._source = self._generate()
 
     def _generate(self):
@@ -373,11 +374,13 @@ class AdjointKernel(object):
         return self.fwd.options()
 
     def key(self):
-        import hashlib
-        h = hashlib.sha256()
-        h.update(self._source.encode())
-        h.update('\0'.join(self.options()).encode())
-        return h.hexdigest()
+        if self._key is None:
+            import hashlib
+            h = hashlib.sha256()
+            h.update(self._source.encode())
+            h.update('\0'.join(self.options()).encode())
+            self._key = h.hexdigest()
+        return self._key
 
 
 class TissueAdjoint(object):
@@ -446,7 +449,7 @@ class TissueAdjoint(object):
         return [v.qname() for v in self.sim._fields]
 
     def _prepare(self):
-        from .simulation import compile_kernel
+        from .simulation import compile_kernel, shared_kernel
         sim = self.sim
         kernel = sim._kernel([])
         be = sim._get_backend(kernel)
@@ -455,25 +458,9 @@ class TissueAdjoint(object):
         akey = (kernel.key(), self.min_blocks, self.threads, self.guards)
         ak = self._generated.get(akey)
         if ak is None:
-            # The trajectory-writing forward kernel has the launch shape,
-            # register cap and tile staging of the simulation's own kernel
-            fwd = _exp.TissueKernel(
-                sim._model, sim._precision, sim._native_math,
-                sim._bound_variables, [], kernel.diffusion, kernel.two_d,
-                list(sim._fields.keys()), sim._rl_states, kernel.block,
-                min_blocks=kernel.min_blocks, math=sim._fp32_math,
-                accumulate=kernel.accumulate,
-                accumulate_states=sim.accumulated_states(), traj=True,
-                stage=kernel.stage, row_pad=kernel.row_pad,
-                stage_lazy=kernel.stage_lazy, sync=kernel.sync,
-                team=kernel.team)
-            threads = self.threads
-            if threads is None and kernel.team:
-                # A resident kernel's CTA is one tile; the reverse kernel's
-                # warps each own tiles: as many warps as there are tiles for
-                # an SM
-                threads = 32 * min(kernel.min_blocks, 8)
-            ak = AdjointKernel(fwd, self.min_blocks, threads, self.guards)
+            ak = shared_kernel(
+                ('adjoint', sim.model_code(), sim._rl) + akey,
+                lambda: self._make(kernel))
             self._generated = {akey: ak}
         key = (id(be), akey, self.segment_steps)
         if self._attached != key:
@@ -482,6 +469,29 @@ class TissueAdjoint(object):
                                            self.segment_steps))
             self._attached = key
         return be
+
+    def _make(self, kernel):
+        """The adjoint kernel of a forward kernel."""
+        sim = self.sim
+        # The trajectory-writing forward kernel has the launch shape,
+        # register cap and tile staging of the simulation's own kernel
+        fwd = _exp.TissueKernel(
+            sim._model, sim._precision, sim._native_math,
+            sim._bound_variables, [], kernel.diffusion, kernel.two_d,
+            list(sim._fields.keys()), sim._rl_states, kernel.block,
+            min_blocks=kernel.min_blocks, math=sim._fp32_math,
+            accumulate=kernel.accumulate,
+            accumulate_states=sim.accumulated_states(), traj=True,
+            stage=kernel.stage, row_pad=kernel.row_pad,
+            stage_lazy=kernel.stage_lazy, sync=kernel.sync,
+            team=kernel.team)
+        threads = self.threads
+        if threads is None and kernel.team:
+            # A resident kernel's CTA is one tile; the reverse kernel's
+            # warps each own tiles: as many warps as there are tiles for an
+            # SM
+            threads = 32 * min(kernel.min_blocks, 8)
+        return AdjointKernel(fwd, self.min_blocks, threads, self.guards)
 
     def forward(self, duration, log_interval=1.0):
         """

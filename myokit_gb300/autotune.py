@@ -68,7 +68,7 @@ def _shipped_path():
 def signature(sim):
     """A string identifying what the best launch shape depends on."""
     import hashlib
-    code = hashlib.sha1(sim._model.code().encode()).hexdigest()[:16]
+    code = hashlib.sha1(sim.model_code().encode()).hexdigest()[:16]
     return '|'.join(str(x) for x in (
         sim._model.name(), code, sim._nx, sim._ny, len(sim._dims),
         sim._precision, sim._accumulate, sim._diffusion_mode(),

@@ -777,6 +777,25 @@ long long blocks_needed(const mkg_sim *s, const mkg_launch *a)
     return (nwt * 32 * split + threads - 1) / threads;
 }
 
+/* Queues the conversion and the copy of the first `rows` log rows of `of`
+ * (this simulation or its partner) to its host buffer, on s's stream */
+int queue_log(mkg_sim *s, mkg_sim *of, int64_t rows)
+{
+    if (of->log_ncol < 1) return MKG_OK;
+    const long long cnt = rows * (long long)of->log_ncol;
+    s->n_launches++;
+    if (of->real == 4)
+        k_log_to_double<float><<<grid_for(cnt), 256, 0, s->stream>>>(
+            (const float *)of->d_log, of->d_log_dbl, cnt);
+    else
+        k_log_to_double<double><<<grid_for(cnt), 256, 0, s->stream>>>(
+            (const double *)of->d_log, of->d_log_dbl, cnt);
+    CK(s, cudaGetLastError());
+    CK(s, cudaMemcpyAsync(of->h_log, of->d_log_dbl, cnt * sizeof(double),
+                          cudaMemcpyDeviceToHost, s->stream));
+    return MKG_OK;
+}
+
 /* Step counters and V words start at zero: before the launches of a chunk,
  * which count its steps from one */
 int reset_step_words(mkg_sim *s)
@@ -1598,6 +1617,13 @@ int mkg_run_chunk(mkg_sim *s, int64_t max_steps, double *t_out,
     CK(s, cudaEventRecord(s->ev1, s->stream));
     CK(s, cudaMemcpyAsync(s->h_status, s->d_status, sizeof(mkg_status),
                           cudaMemcpyDeviceToHost, s->stream));
+    /* The chunk's log rows behind its launches, before the one
+     * synchronisation (after a halt or an error those not written are not
+     * used; a frame buffer keeps its rows on the device) */
+    if (rows > 0) {
+        if (!s->frame_buf && (r = queue_log(s, s, rows))) return r;
+        if (p && (r = queue_log(s, p, rows))) return r;
+    }
     CK(s, cudaStreamSynchronize(s->stream));
     if (s->h_status->error == MKG_DEV_LAUNCH) {
         s->running = false;
@@ -1625,38 +1651,9 @@ int mkg_run_chunk(mkg_sim *s, int64_t max_steps, double *t_out,
     int64_t rows_done = 0;
     for (int64_t i = 0; i < done; ++i)
         if (s->h_steps[i].log_row >= 0) rows_done = s->h_steps[i].log_row + 1;
-    if (s->frame_buf) {
-        /* Frames stay on the device */
-        s->frame_next += rows_done;
-    } else if (rows_done > 0 && s->log_ncol > 0) {
-        const long long cnt = rows_done * (long long)s->log_ncol;
-        s->n_launches++;
-        if (s->real == 4)
-            k_log_to_double<float><<<grid_for(cnt), 256, 0, s->stream>>>(
-                (const float *)s->d_log, s->d_log_dbl, cnt);
-        else
-            k_log_to_double<double><<<grid_for(cnt), 256, 0, s->stream>>>(
-                (const double *)s->d_log, s->d_log_dbl, cnt);
-        CK(s, cudaGetLastError());
-        CK(s, cudaMemcpyAsync(s->h_log, s->d_log_dbl, cnt * sizeof(double),
-                              cudaMemcpyDeviceToHost, s->stream));
-    }
-    if (p && rows_done > 0 && p->log_ncol > 0) {
-        /* The partner's rows, through the same stream */
-        const long long cnt = rows_done * (long long)p->log_ncol;
-        s->n_launches++;
-        if (p->real == 4)
-            k_log_to_double<float><<<grid_for(cnt), 256, 0, s->stream>>>(
-                (const float *)p->d_log, p->d_log_dbl, cnt);
-        else
-            k_log_to_double<double><<<grid_for(cnt), 256, 0, s->stream>>>(
-                (const double *)p->d_log, p->d_log_dbl, cnt);
-        CK(s, cudaGetLastError());
-        CK(s, cudaMemcpyAsync(p->h_log, p->d_log_dbl, cnt * sizeof(double),
-                              cudaMemcpyDeviceToHost, s->stream));
-    }
+    /* Frames stay on the device */
+    if (s->frame_buf) s->frame_next += rows_done;
     if (p) p->last_rows = rows_done;
-    CK(s, cudaStreamSynchronize(s->stream));
     float ms = 0;
     cudaEventElapsedTime(&ms, s->ev0, s->ev1);
     s->last_ms = ms;

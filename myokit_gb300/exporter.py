@@ -792,6 +792,7 @@ class TissueKernel(object):
         # Single precision: variables computed by the trigonometric cubic
         # formula, refined by mkg_cubic_root: name -> (b, c, d) names
         self.cubic = {}
+        self._key = None
         self._source = self._generate()
         if self.team and asked:
             # The resident tile's shared memory, where staging was asked for
@@ -1733,10 +1734,12 @@ class TissueKernel(object):
 
     def key(self):
         """A hash identifying the source and options, for the cubin cache."""
-        h = hashlib.sha256()
-        h.update(self._source.encode())
-        h.update('\0'.join(self.options()).encode())
-        return h.hexdigest()
+        if self._key is None:
+            h = hashlib.sha256()
+            h.update(self._source.encode())
+            h.update('\0'.join(self.options()).encode())
+            self._key = h.hexdigest()
+        return self._key
 
     def bytes_per_cell_step(self):
         """

@@ -27,6 +27,28 @@ _CUBIN_CACHE = {}
 _CUBIN_LOCK = threading.Lock()
 
 
+# Generated kernels by what they are generated from (the model's code and
+# every option), so that simulations of one model generate them once; the
+# least recently used of more than 32 is dropped
+_KERNELS = OrderedDict()
+_KERNELS_LOCK = threading.Lock()
+
+
+def shared_kernel(key, generate):
+    """The kernel of ``key``, generated unless it was before."""
+    with _KERNELS_LOCK:
+        k = _KERNELS.get(key)
+        if k is not None:
+            _KERNELS.move_to_end(key)
+            return k
+    k = generate()
+    with _KERNELS_LOCK:
+        _KERNELS[key] = k
+        while len(_KERNELS) > 32:
+            _KERNELS.popitem(last=False)
+    return k
+
+
 def _cache_dir():
     d = os.environ.get('MYOKIT_GB300_CACHE')
     if d is None:
@@ -230,6 +252,9 @@ class SimulationCUDA(object):
         self._gy_field = None
         self._g_arrays = None      # (key, gx, gy) arrays of the above
         self._connections = None
+        self._c_arrays = None      # cells and conductances of the connections
+        self._code = None           # (model version, the model's code)
+        self._log_plan = None       # columns of the last log (_log_columns)
         self._paced_cells = None
         if self._diffusion_enabled:
             self.set_paced_cells()
@@ -434,6 +459,7 @@ class SimulationCUDA(object):
                 raise ValueError('Invalid conductance: ' + str(c))
             conns.append((i, j, c))
         self._connections = conns
+        self._c_arrays = None
         self._gx_field = self._gy_field = None
         self._g_arrays = None
 
@@ -884,6 +910,12 @@ class SimulationCUDA(object):
         self._tune_sig = None
         return best
 
+    def model_code(self):
+        """The code of the simulation's model (kept per model version)."""
+        if self._code is None or self._code[0] != self._model_version:
+            self._code = (self._model_version, self._model.code())
+        return self._code[1]
+
     def accumulated_states(self):
         """The states accumulated in FP64 or with a compensated update."""
         if self._accumulate is None:
@@ -960,14 +992,17 @@ class SimulationCUDA(object):
             tuple(v.qname() for v in inter_log))
         k = self._kernels.get(key)
         if k is None:
-            k = _exp.TissueKernel(
-                self._model, self._precision, self._native_math,
-                self._bound_variables, inter_log, mode, two_d,
-                list(self._fields.keys()), self._rl_states, block,
-                min_blocks=minb, math=self._fp32_math,
-                accumulate=self._accumulate, accumulate_states=acc,
-                stage=stage, row_pad=row_pad, stage_lazy=lazy,
-                sync=self._sync_mode(), split=split, team=team)
+            # (two models with the same code give the same kernel)
+            k = shared_kernel(
+                ('step', self.model_code(), self._rl) + key[:1] + key[2:],
+                lambda: _exp.TissueKernel(
+                    self._model, self._precision, self._native_math,
+                    self._bound_variables, inter_log, mode, two_d,
+                    list(self._fields.keys()), self._rl_states, block,
+                    min_blocks=minb, math=self._fp32_math,
+                    accumulate=self._accumulate, accumulate_states=acc,
+                    stage=stage, row_pad=row_pad, stage_lazy=lazy,
+                    sync=self._sync_mode(), split=split, team=team))
             if len(self._kernels) > 16:
                 self._kernels.clear()
             self._kernels[key] = k
@@ -1013,6 +1048,10 @@ class SimulationCUDA(object):
         Maps every log key to a column source: ``('time',)``, ``('pace',)``
         or a per-cell ``(item, cell)`` pair (openclsim.c:916-1001).
         """
+        # (the columns of a log with the same keys are those of the last)
+        asked = (tuple(log.keys()), kernel.key(), self._diffusion_enabled)
+        if self._log_plan is not None and self._log_plan[0] == asked:
+            return self._log_plan[1]
         tvar = self._model.binding('time')
         pvar = self._model.binding('pace')
         tname = None if tvar is None else tvar.qname()
@@ -1058,6 +1097,7 @@ class SimulationCUDA(object):
                 raise Exception(
                     'Unknown variables found in logging dictionary.')
             sources.append((item, cell))
+        self._log_plan = (asked, sources)
         return sources
 
     def _prepare_log(self, log, global_vars):
@@ -1200,10 +1240,14 @@ class SimulationCUDA(object):
             be.check(lib.mkg_set_conductance_field(
                 h, _lib.dptr(gx), gx.size, _lib.dptr(gy), gy.size))
         elif mode == _exp.DIFF_CONN:
-            c = np.array(self._connections, dtype=float).reshape(-1, 3)
-            c1 = np.ascontiguousarray(c[:, 0].astype(np.int64))
-            c2 = np.ascontiguousarray(c[:, 1].astype(np.int64))
-            gg = np.ascontiguousarray(c[:, 2])
+            # Converted once per set_connections
+            if self._c_arrays is None:
+                c = np.array(self._connections, dtype=float).reshape(-1, 3)
+                self._c_arrays = (
+                    np.ascontiguousarray(c[:, 0].astype(np.int64)),
+                    np.ascontiguousarray(c[:, 1].astype(np.int64)),
+                    np.ascontiguousarray(c[:, 2]))
+            c1, c2, gg = self._c_arrays
             be.check(lib.mkg_set_connections(
                 h, _lib.i64ptr(c1), _lib.i64ptr(c2), _lib.dptr(gg), len(gg)))
         if not self._diffusion_enabled:
@@ -1239,10 +1283,14 @@ class SimulationCUDA(object):
         items = np.ascontiguousarray([c[0] for c in cols], dtype=np.int32)
         cells = np.ascontiguousarray([c[1] for c in cols], dtype=np.int64)
         logging_states = any(c[0] < self._nstate for c in cols)
-        be.log_sig = None
-        be.check(lib.mkg_set_log(
-            h, _lib.i32ptr(items), _lib.i64ptr(cells), len(cols),
-            1 if logging_states else 0))
+        # The columns a handle was last given stay on the device
+        sig = ('log', items.tobytes(), cells.tobytes(), logging_states)
+        if be.log_sig != sig:
+            be.log_sig = None
+            be.check(lib.mkg_set_log(
+                h, _lib.i32ptr(items), _lib.i64ptr(cells), len(cols),
+                1 if logging_states else 0))
+            be.log_sig = sig
         be.check(lib.mkg_set_tuning(h, self._launch_steps(),
                                     self._blocks_per_sm, self._graphs))
         be.check(lib.mkg_run_begin(h, tmin, tmax, self._step_size,
@@ -1326,14 +1374,19 @@ class SimulationCUDA(object):
         if chunks_t:
             tt = np.concatenate(chunks_t)
             pp = np.concatenate(chunks_p)
-            vv = np.concatenate(chunks_v) if ncol else None
+            # One row per column, in the precision of the log's arrays
+            dt = np.float32 if self._precision == myokit.SINGLE_PRECISION \
+                else np.float64
+            tt, pp = tt.astype(dt), pp.astype(dt)
+            vv = np.ascontiguousarray(
+                np.concatenate(chunks_v).T, dtype=dt) if ncol else None
             for key, src, c in zip(keys, sources, col_of_key):
                 if src[0] == 'time':
                     data = tt
                 elif src[0] == 'pace':
                     data = pp
                 else:
-                    data = vv[:, c]
+                    data = vv[c]
                 _extend(log[key], data)
         return status == _lib.MKG_HALT_NAN
 
@@ -1474,6 +1527,8 @@ def _extend(target, values):
     """Appends numpy values to a log list or array."""
     if isinstance(target, array.array):
         dt = np.float32 if target.typecode == 'f' else np.float64
-        target.frombytes(np.ascontiguousarray(values, dtype=dt).tobytes())
+        if values.dtype != dt:
+            values = values.astype(dt)
+        target.frombytes(values.tobytes())
     else:
         target.extend(np.asarray(values, dtype=float).tolist())
