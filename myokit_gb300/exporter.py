@@ -536,7 +536,8 @@ def _pow_helpers(single, outline=False):
     out.append('static __device__ __forceinline__ Real mkg_pow1p5(Real x)'
                f' {{ return x * {sq}(x); }}')
     if single:
-        out.extend([_EXP_HELPER, _CUBIC_HELPER])
+        out.extend([_EXP_HELPER, _CUBIC_HELPER.replace(
+            '__forceinline__', '__noinline__') if outline else _CUBIC_HELPER])
     return '\n'.join(out)
 
 
@@ -792,6 +793,9 @@ class TissueKernel(object):
         # Single precision: variables computed by the trigonometric cubic
         # formula, refined by mkg_cubic_root: name -> (b, c, d) names
         self.cubic = {}
+        # Functions that several equations call, and the calls by name
+        self.functions = []
+        self.repeated = {}
         self._key = None
         self._source = self._generate()
         if self.team and asked:
@@ -911,7 +915,7 @@ class TissueKernel(object):
             refs = set(self._name(r) for r in rhs.references())
             if self.team:
                 c = _teams.cost(rhs, self.single) + (
-                    30 if self._name(lhs) in self.cubic else 0)
+                    _teams.CUBIC if self._name(lhs) in self.cubic else 0)
             else:
                 c = OpCensus()
                 c.add(rhs)
@@ -1061,18 +1065,21 @@ class TissueKernel(object):
                 else:
                     rhs = fold(eq.rhs)
                 self.rhs_eqs.append((eq.lhs, rhs))
-                self.census.add(rhs)
-                name = self._name(eq.lhs)
-                if self.single and isinstance(eq.lhs, myokit.Name):
-                    bcd = cubic_root_coefficients(rhs)
-                    if bcd is not None:
-                        self.cubic[name] = tuple(self._name(r) for r in bcd)
-                        self.census.arith += 20
-                line = f'{tab}const Real {name} = {self.rhs_code(eq.lhs, rhs)};'
-                body.append(line)
-                item(eq.lhs, rhs, line)
-                defined.add(name)
-                flush()
+        if self.team > 1 and self.single:
+            self._find_repeated()
+        for lhs, rhs in self.rhs_eqs:
+            self.census.add(rhs)
+            name = self._name(lhs)
+            if self.single and isinstance(lhs, myokit.Name):
+                bcd = cubic_root_coefficients(rhs)
+                if bcd is not None:
+                    self.cubic[name] = tuple(self._name(r) for r in bcd)
+                    self.census.arith += 20
+            line = f'{tab}const Real {name} = {self.rhs_code(lhs, rhs)};'
+            body.append(line)
+            item(lhs, rhs, line)
+            defined.add(name)
+            flush()
         if len(emitted) != len(updates):   # pragma: no cover
             raise ValueError('Could not order the state updates.')
         self._inter_names = [self._name(v) for v in self.inter_log]
@@ -1305,8 +1312,21 @@ class TissueKernel(object):
                 f'{tab}    if (live) {{', log_b, f'{tab}    }}',
                 f'{tab}    }}']
 
-        out = []
+        # When the neighbours' V is asked for: its words are there about 500
+        # cycles into a step, and a word asked for before that is asked for
+        # again where it is needed, a trip to L2 of 880 cycles; one asked for
+        # at the first meeting may not be back yet. So at the start of a step
+        # whose first phase is shorter than that trip (an addition counts as
+        # 5 cycles in single precision, 67 in double), and at the end of a
+        # longer one, which the wait is then hidden behind. us per step asked
+        # for at the start, before and after the first meeting: 48 states,
+        # 61 x 47 cells (1740 cycles) 1.64, 1.57, 1.61, 128 x 128 2.00, 1.91,
+        # 1.91; 8 states, 200 cells (390 cycles) 0.55, 0.60, 0.62, double
+        # precision (3500) 2.59, 2.58, 2.80.
         nphase = len(team.work)
+        ask_late = nphase > 1 and \
+            max(team.cost[0]) > 880 / (5 if self.single else 67)
+        out = []
         for p in range(self.team):
             gate_list = [i for f in range(nphase) for i in team.gates_of[f][p]]
             names = set()
@@ -1329,12 +1349,16 @@ class TissueKernel(object):
                 take = [f'{tab}    const Real {_IDIFF} = 0;',
                         f'{tab}    (void){_IDIFF};']
             early = p in halo and team.halo_early[p]
+            if p in halo and (early or not ask_late):
+                out.append(f'{tab}    MKG_HALO_ASK()')
             if early:
                 out.extend(take)
             if p == 0:
                 # Logged values, before any state changes; a NaN halt
                 out.append(f'{tab}    if (row >= 0) {{')
                 if not early:
+                    if halo and ask_late:
+                        out.append(f'{tab}    MKG_HALO_ASK()')
                     out.extend(take)
                 out.append(f'{tab}    if (live) {{')
                 out.append(log)
@@ -1344,6 +1368,8 @@ class TissueKernel(object):
                 out.append(f'{tab}    MKG_CHECK_HALT()')
             after = []           # stores that wait for the team's loads
             for f in range(nphase):
+                if f == 1 and p in halo and ask_late and not early:
+                    out.append(f'{tab}    MKG_HALO_ASK()')
                 if f:
                     out.append(f'{tab}    mkg_team_sync();')
                 if f == 1:
@@ -1353,10 +1379,15 @@ class TissueKernel(object):
                 for x in team.read[f][p]:
                     out.append(f'{tab}    const Real {x} = '
                                f'hs[{team.slots[x]}][lane];')
-                if f == nphase - 1 and (p in halo or (p == 0 and not halo)) \
-                        and not early and (team.halo[p] or p == 0):
+                late = f == nphase - 1 and not early and (
+                    team.halo[p] or p == 0)
+                for x in team.work[f][p]:
+                    if late and _IDIFF in refs[x]:
+                        out.extend(take)
+                        late = False
+                    out.append(line_of[x])
+                if late:
                     out.extend(take)
-                out.extend(line_of[x] for x in team.work[f][p])
                 for x in team.written[f][p]:
                     out.append(f'{tab}    hs[{team.slots[x]}][lane] = {x};')
                 for i in team.gates_of[f][p]:
@@ -1413,9 +1444,11 @@ class TissueKernel(object):
             # took 42 us a step, with both called 20 us; 304 tiles 82 and 29
             # us. A small model's code fits: Beeler-Reuter (2600 instructions
             # of them) 4.0 us inlined, 4.2 us called.
-            '@POW_HELPERS@': _pow_helpers(
+            '@POW_HELPERS@': '\n'.join([_pow_helpers(
                 self.single, 75 * self.census.trans +
-                65 * self.census.divide > 6000),
+                65 * self.census.divide > 6000 if not self.single
+                else self.team > 1 and len(self.cubic) > 1)] +
+                self.functions),
             '@NEED_HALO@': ' || '.join(f'part_ == {p}' for p in halo)
             or 'false',
                     }
@@ -1699,10 +1732,46 @@ class TissueKernel(object):
             return w.scaled_exp(x, -1.0)
         return f'{w._fn("exp")}(-({x}))'
 
+    def _find_repeated(self):
+        """
+        Equations that differ only in the variables they refer to (the same
+        buffer in several compartments) become calls of one function: a
+        resident tile's code runs from a 32 KB instruction cache.
+        """
+        def shape(e, refs):
+            if isinstance(e, (myokit.Name, myokit.Derivative)):
+                if e not in refs:
+                    refs.append(e)
+                return refs.index(e)
+            if isinstance(e, myokit.Number):
+                return float(e.eval())
+            return (type(e).__name__,) + tuple(shape(x, refs) for x in e)
+
+        found = {}
+        for lhs, rhs in self.rhs_eqs:
+            if _teams.cost(rhs, self.single) >= 60:
+                refs = []
+                key = repr(shape(rhs, refs))
+                found.setdefault(key, []).append((lhs, rhs, refs))
+        for equations in found.values():
+            if len(equations) < 2:
+                continue
+            name = 'mkg_equation_%d' % len(self.functions)
+            _, rhs, refs = equations[0]
+            self.writer.set_lhs_function(lambda x: 'a%d' % refs.index(x))
+            self.functions.append(
+                f'static __device__ __noinline__ Real {name}('
+                + ', '.join(f'Real a{i}' for i in range(len(refs)))
+                + f')\n{{\n    return {self.writer.ex(rhs)};\n}}')
+            self.writer.set_lhs_function(self._name)
+            for lhs, _, refs in equations:
+                self.repeated[self._name(lhs)] = name + '(' + ', '.join(
+                    self._name(r) for r in refs) + ')'
+
     def rhs_code(self, lhs, rhs):
         """CUDA expression for an equation's right-hand side, with the
         cubic root refinement where it applies."""
-        text = self.writer.ex(rhs)
+        text = self.repeated.get(self._name(lhs)) or self.writer.ex(rhs)
         bcd = self.cubic.get(self._name(lhs))
         if bcd is not None:
             text = f'mkg_cubic_root({text}, {bcd[0]}, {bcd[1]}, {bcd[2]})'

@@ -22,11 +22,13 @@ from ._deps import myokit
 # Double precision: an addition waits 67 cycles for the double precision
 # pipe; exp and division run on the integer pipes (csrc/mkg_math64.h).
 _COST = {
-    True: {'div': 5, 'exp': 5, 'log': 16, 'sqrt': 11, 'trig': 20, 'pow': 25,
-           'cond': 1, 'rl': 10},
+    True: {'div': 3, 'exp': 3, 'log': 20, 'sqrt': 14, 'trig': 25, 'pow': 28,
+           'cond': 1, 'rl': 6},
     False: {'div': 4, 'exp': 6, 'log': 7, 'sqrt': 5, 'trig': 22, 'pow': 14,
             'cond': 1, 'rl': 9},
 }
+# The refinement of a cubic root (single precision)
+CUBIC = 55
 # Intermediate variables this cheap are evaluated where they are used
 # rather than handed over
 _CHEAP = 1

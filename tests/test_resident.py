@@ -93,6 +93,44 @@ def test_plan(decker, br77, team, rl, precision, kw):
                        for c in k.team_plan.cost)
 
 
+@pytest.mark.parametrize('team', [1, 2, 4])
+def test_equations_that_are_alike(decker, team):
+    # The three calcium buffers are one function, called with the
+    # arguments of each (a single warp has its code to itself)
+    k = _kernel(decker, SP, team, True)
+    names = ['ca_cal', 'ca_i', 'ca_jsr']
+    calls = [k.repeated.get('v_' + n) for n in names]
+    if team == 1:
+        assert not k.functions and not any(calls)
+        return
+    assert len(k.functions) == 1 and ' mkg_equation_0(' in k.functions[0]
+    text = k.source()
+    for n, call in zip(names, calls):
+        assert call == 'mkg_equation_0(%s)' % ', '.join(
+            'v_%s_%s' % (n, x) for x in 'bcd')
+        assert text.count(call) >= 1
+
+
+def test_when_neighbours_are_asked(decker, br77):
+    # At the start of a step whose first phase is short, at the end of a
+    # long first phase, and where one warp does all at the start
+    for m, rl, precision, team, late in (
+            (decker, True, SP, 4, True), (decker, True, SP, 1, False),
+            (br77, False, SP, 4, False), (br77, False, DP, 8, True)):
+        body = _kernel(m, precision, team, rl).team_body
+        first = body.index('const Real', body.index('part_ == 0'))
+        asks = [i for i in range(len(body))
+                if body.startswith('MKG_HALO_ASK()', i)]
+        meets = body.index('mkg_team_sync();')
+        log = body.index('if (row >= 0)')
+        assert asks and first < asks[0]
+        if late:
+            assert log < asks[0] and asks[-1] > asks[0]
+            assert body[asks[1]:meets].count('\n') == 1
+        else:
+            assert asks[0] < log
+
+
 @pytest.mark.parametrize('precision', [SP, DP])
 def test_compiles(decker, precision):
     k = _kernel(decker, precision, 16, True)
