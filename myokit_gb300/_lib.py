@@ -122,6 +122,9 @@ SIGNATURES = {
         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64]),
     'mkg_adj_attach': (ctypes.c_int, [
         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int32]),
+    'mkg_adj_attach_map': (ctypes.c_int, [
+        ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int32,
+        ctypes.c_int32, ctypes.c_int32]),
     'mkg_adj_forward': (ctypes.c_int, [
         ctypes.c_void_p, ctypes.c_double, ctypes.c_double, ctypes.c_double,
         ctypes.c_double, _c_int64_p]),

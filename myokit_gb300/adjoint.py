@@ -29,8 +29,16 @@ import numpy as np
 from ._deps import myokit
 from . import exporter as _exp
 from . import _lib
+from . import autotune
 
 _N = myokit.Number
+# Tiles per SM up to which the reverse goes by tape and sweep, where the
+# sweep's registers allow it. ms forward and backward, general and so: 8
+# states, double precision, 200 steps: 2 tiles in all 9.9, 2.0; 100 steps: one
+# tile per SM 6.0, 2.7; four 6.6, 4.4; eight 8.9, 8.1. Single precision, 100
+# steps: four 1.45, 1.25; eight 1.78, 1.61; ten 1.90, 1.91. 48 states, single
+# precision, 100 steps: one 2.42, 1.94; three (all that fit) 3.15, 2.89.
+_MAP_TILES = 8
 
 
 def _mul(a, b):
@@ -190,7 +198,8 @@ class AdjointKernel(object):
     (homogeneous or per-edge conductances on a 1D or 2D grid, arbitrary
     connections, none) and scalar fields.
     """
-    def __init__(self, fwd, min_blocks=1, threads=None, guards=True):
+    def __init__(self, fwd, min_blocks=1, threads=None, guards=True,
+                 tiles_per_sm=0):
         self.fwd = fwd
         self.single = fwd.single
         self.min_blocks = int(min_blocks)
@@ -199,7 +208,31 @@ class AdjointKernel(object):
             raise ValueError('threads must be a multiple of 32 up to 1024')
         self.guards = bool(guards)
         self._key = None
-        self._source = self._generate()
+        # Numbers per cell and step on the tape, and warps per tile of the
+        # sweep (0: the general reverse kernel)
+        self.slots = self.parts = 0
+        self._source = self._generate_map(tiles_per_sm) \
+            if tiles_per_sm else None
+        if self._source is None:
+            self._source = self._generate()
+
+    def _forward_values(self, tab):
+        """The model's variables at step k, from the trajectory."""
+        fwd = self.fwd
+        name = fwd._name
+        fw = []
+        for i, s in enumerate(fwd.states):
+            fw.append(f'{tab}const Real {name(s)} = xk[(long long){i}'
+                      f' * pitch + cid];')
+        for k, var in enumerate(fwd.fields):
+            fw.append(f'{tab}const Real {name(var)} = '
+                      f'field[(long long){k} * pitch + cid];')
+        for lhs, rhs in fwd.cell_const_eqs:
+            fw.append(f'{tab}const Real {name(lhs)} = {fwd.writer.ex(rhs)};')
+        for lhs, rhs in fwd.rhs_eqs:
+            fw.append(f'{tab}const Real {name(lhs)} = '
+                      f'{fwd.rhs_code(lhs, rhs)};')
+        return fw
 
     def _generate(self):
         fwd = self.fwd
@@ -207,19 +240,7 @@ class AdjointKernel(object):
         name = fwd._name
         tab = '            '
         states = fwd.states
-        # Forward values at step k, from the trajectory
-        fw = []
-        for i, s in enumerate(states):
-            fw.append(f'{tab}const Real {name(s)} = xk[(long long){i}'
-                      f' * pitch + cid];')
-        for k, var in enumerate(fwd.fields):
-            fw.append(f'{tab}const Real {name(var)} = '
-                      f'field[(long long){k} * pitch + cid];')
-        for lhs, rhs in fwd.cell_const_eqs:
-            fw.append(f'{tab}const Real {name(lhs)} = {w.ex(rhs)};')
-        for lhs, rhs in fwd.rhs_eqs:
-            fw.append(f'{tab}const Real {name(lhs)} = '
-                      f'{fwd.rhs_code(lhs, rhs)};')
+        fw = self._forward_values(tab)
 
         # Adjoint accumulators: every state, field, per-cell constant,
         # equation left-hand side and the diffusion current
@@ -360,6 +381,329 @@ class AdjointKernel(object):
         # The forward kernel with trajectory output, in the same module
         return self._join(fwd.source(), text)
 
+    def _step_matrix(self, tab):
+        """
+        ``(partials, rows, entries)``: the code of the local partial
+        derivatives and of the rows of the matrix of one step, and per
+        column name the ``(state, slot)`` of its entries. A forward Euler
+        state's row is the identity plus its entries.
+        """
+        fwd = self.fwd
+        w = fwd.writer
+        name = fwd._name
+        states = fwd.states
+        equations = fwd.cell_const_eqs + fwd.rhs_eqs
+        leaves = [name(s) for s in states] + \
+            [name(v) for v in fwd.fields] + [_exp._IDIFF]
+        known = set(leaves) | set(name(lhs) for lhs, _ in equations)
+        partials = []
+        local = {}               # name -> [(referenced name, factor)]
+        for lhs, rhs in equations:
+            n = name(lhs)
+            local[n] = []
+            bcd = fwd.cubic.get(n)
+            if bcd is not None:
+                # A refined root x of x^3 + b x^2 + c x + d (see _generate)
+                b, c, d = bcd
+                g = w.fma(w.fma('2', b, f'3 * {n}'), n, c)
+                r = f'r_{n}'
+                one = '-1 / g_' if self.single else 'mkg_div(-1.0, g_)'
+                partials.append(f'{tab}Real {r};')
+                partials.append(f'{tab}{{ const Real g_ = {g}; {r} = '
+                                f'g_ != 0 ? {one} : (Real)0; }}')
+                for x, p in ((b, f'{r} * {n} * {n}'), (c, f'{r} * {n}'),
+                             (d, r)):
+                    if x in known:
+                        local[n].append((x, f'({p})'))
+                continue
+            for r in _references(rhs):
+                rn = name(r)
+                if rn not in known:
+                    continue
+                dp = local_partial(rhs, r)
+                if dp is None:
+                    continue
+                if isinstance(dp, _N):
+                    local[n].append((rn, float(dp.eval())))
+                    continue
+                if isinstance(dp, myokit.PrefixMinus) and \
+                        isinstance(dp[0], _N):
+                    local[n].append((rn, -float(dp[0].eval())))
+                    continue
+                p = f'p_{len(partials)}'
+                partials.append(f'{tab}const Real {p} = {w.ex(dp)};')
+                local[n].append((rn, p))
+
+        def ref(var):
+            x = fwd.literal_subst.get(myokit.Name(var))
+            return w.ex(x) if x is not None else name(var)
+
+        rows = []
+        entries = {}             # column -> [(state, slot)]
+        slots = 0
+        order = [name(lhs) for lhs, _ in equations]
+        for i, s in enumerate(states):
+            acc = {}
+
+            def add(rn, a, p=1.0):
+                if isinstance(p, float) and abs(p) != 1.0:
+                    p = f'(Real){p!r}'
+                if isinstance(p, float):
+                    a = a if p > 0 else f'-{a}'
+                    if rn in acc:
+                        rows.append(f'{tab}    {acc[rn]} += {a};')
+                        return
+                elif rn in acc:
+                    rows.append(f'{tab}    {acc[rn]} = '
+                                f'{w.fma(a, p, acc[rn])};')
+                    return
+                else:
+                    a = f'{a} * {p}'
+                acc[rn] = 'J_' + rn
+                rows.append(f'{tab}    Real J_{rn} = {a};')
+
+            rows.append(f'{tab}{{')
+            n = name(s)
+            if s in fwd.rl_states:
+                inf, tau = fwd.rl_states[s]
+                ri, rt = ref(inf), ref(tau)
+                rows.append(f'{tab}    const Real E_ = '
+                            f'{fwd.decay(tau, rt, fwd.rates)};')
+                add(n, 'E_')
+                if name(inf) in known and \
+                        myokit.Name(inf) not in fwd.literal_subst:
+                    add(name(inf), '(1 - E_)')
+                if name(tau) in known and \
+                        myokit.Name(tau) not in fwd.literal_subst:
+                    num = f'-({ri} - {n}) * E_ * dt_'
+                    den = f'{rt} * {rt}'
+                    q = f'{num} / ({den})' if self.single else \
+                        f'mkg_div({num}, {den})'
+                    add(name(tau), q)
+            else:
+                add(name(s.lhs()), 'dt_')
+            for x in reversed(order):
+                if x in acc:
+                    for rn, p in local[x]:
+                        add(rn, acc[x], p)
+            for x in leaves:
+                if x in acc:
+                    rows.append(f'{tab}    tape[{slots} * 32] = {acc[x]};')
+                    entries.setdefault(x, []).append((i, slots))
+                    slots += 1
+            rows.append(f'{tab}}}')
+        return partials, rows, entries, slots
+
+    def _generate_map(self, tiles_per_sm):
+        """
+        The tape and sweep kernels (``csrc/adjoint_map.cu.in``) for a
+        resident simulation with that many tiles on an SM, or None where
+        the sweep's tiles would not fit.
+        """
+        fwd = self.fwd
+        w = fwd.writer
+        name = fwd._name
+        tab = '    '
+        states = fwd.states
+        vm = fwd.i_vm
+        if not fwd.team or vm < 0:
+            return None
+        partials, rows, entries, x0 = self._step_matrix(tab)
+        diff = fwd.diffusion
+        extra = {_exp.DIFF_NONE: 0, _exp.DIFF_GRID: 2 if fwd.two_d
+                 else 1, _exp.DIFF_HETERO: 4 if fwd.two_d else 2,
+                 _exp.DIFF_CONN: 5}[diff]
+        self.slots = x0 + extra
+
+        cols = [(name(s), j, None) for j, s in enumerate(states)]
+        cols += [(name(v), None, k) for k, v in enumerate(fwd.fields)]
+        current = entries.get(_exp._IDIFF, []) if diff else []
+
+        def price(c):
+            return 2 + 2 * len(entries.get(c[0], ()))
+        words = 1 if self.single else 2
+        shared = (2 * len(states) + 2) * 32 * 4 * words + 32
+        for parts in (4, 2) if self.single else (8, 4, 2):
+            # Columns to warps: V's, which the next step waits for, to the
+            # first, the conductances' gradients to the last
+            load = [0.0] * parts
+            mine = [[] for _ in range(parts)]
+            load[0] += 10 + 2 * len(current) + price(cols[vm])
+            mine[0].append(cols[vm])
+            load[-1] += 2 * extra
+            for c in sorted((c for c in cols if c[1] != vm),
+                            key=lambda c: (-price(c), c[0])):
+                p = min(range(parts), key=load.__getitem__)
+                mine[p].append(c)
+                load[p] += price(c)
+            # Registers of a thread: the numbers of two steps, and some
+            held = [[t for c in mine[p] for _, t in entries.get(c[0], ())] +
+                    ([t for _, t in current] if p == 0 else []) +
+                    (list(range(x0, x0 + extra)) if p == parts - 1 else [])
+                    for p in range(parts)]
+            need = words * (2 * max(len(h) for h in held) + 16) + 40
+            if need <= 255 and 32 * parts * tiles_per_sm * need <= 65536 \
+                    and tiles_per_sm * (shared + 1024) <= 227 * 1024:
+                break
+        else:
+            return None
+        # (rows of the current besides V's wait for the other warps)
+        meet_twice = any(i != vm for i, _ in current)
+        self.parts = parts
+
+        def step(p, cur, nxt, a):
+            out = []
+            o = lambda x: out.append(f'{tab * 3}{x}')  # noqa: E731
+            o('if (s + 1 < n) tape -= back;')
+            for q, t in enumerate(held[p]):
+                o(f'{nxt}{q} = __ldcg(tape + {t} * 32);')
+            at = {t: f'{cur}{q}' for q, t in enumerate(held[p])}
+            if p == 0:
+                # (a log row is known two steps ahead, its gradient one)
+                o('const Real loss_ = next_;')
+                o('next_ = row_ >= 0 && col_ >= 0 ? lgrad[(long long)row_ *'
+                  ' b.nprobe + col_] : (Real)0;')
+                o('row_ = s + 2 < n ? a.steps[n - 3 - s].log_row : -1;')
+                lv = f'ls[{a}][{vm}][lane]'
+                if diff:
+                    o('MKG_GATHER(mu_)')
+                    o(f'const Real l{vm}_ = {lv} + gather;')
+                    o(f'{lv} = l{vm}_;')
+                    o('mu_ = 0;')
+                    for i, t in current:
+                        x = f'l{vm}_' if i == vm else f'ls[{a}][{i}][lane]'
+                        o(f'mu_ = {w.fma(x, at[t], "mu_")};')
+                    o('MKG_PUBLISH(mu_)')
+                    o(f'ms[{a}][lane] = mu_;')
+                else:
+                    o(f'const Real l{vm}_ = {lv};')
+            o('mkg_parts_sync();')
+            o(f'if (s_stop[{a}]) break;')
+            rows_needed = sorted(set(
+                i for c in mine[p] for i, _ in entries.get(c[0], ())) | set(
+                c[1] for c in mine[p] if c[1] is not None and
+                states[c[1]] not in fwd.rl_states))
+            for i in rows_needed:
+                if p or i != vm:
+                    o(f'const Real l{i}_ = ls[{a}][{i}][lane];')
+            for c, j, k in mine[p]:
+                own = j is not None and states[j] not in fwd.rl_states
+                start = f'l{j}_' if own else '(Real)0'
+                o(f'{{ Real a_ = {start}, b_ = 0;')
+                for q, (i, t) in enumerate(entries.get(c, ())):
+                    x = 'ab'[q & 1] + '_'
+                    o(f'  {x} = {w.fma(f"l{i}_", at[t], x)};')
+                o('  a_ += b_;')
+                if j == vm:
+                    o('  a_ += loss_;')
+                    if diff:
+                        o('  a_ += mu_ * cdiag;')
+                if j is None:
+                    o(f'  f{k}_ += a_; }}')
+                else:
+                    o(f'  ls[{1 - a}][{j}][lane] = a_; }}')
+            if p == parts - 1 and diff:
+                x = [at[x0 + q] for q in range(extra)]
+                o(f'const Real mu_ = ms[{a}][lane];')
+                if diff == _exp.DIFF_GRID:
+                    o(f'gx_ += mu_ * {x[0]};')
+                    if fwd.two_d:
+                        o(f'gy_ += mu_ * {x[1]};')
+                elif diff == _exp.DIFF_HETERO:
+                    o(f'gx_ += mu_ * ({x[0]} + {x[1]});')
+                    if fwd.two_d:
+                        o(f'gy_ += mu_ * ({x[2]} + {x[3]});')
+                    for q in range(extra):
+                        o(f'e{q}_ += (double)mu_ * (double){x[q]};')
+                else:
+                    o(f'gx_ += mu_ * {x[4]};')
+                    for q in range(4):
+                        o(f'e{q}_ += (double)mu_ * (double){x[q]};')
+                    o('if (p0_ + 4 < p1_) {')
+                    o('  const Real *vk = (const Real *)b.traj + (long long)'
+                      f'((n - 1 - s) * N_STATE + {vm}) * pitch;')
+                    o('  const Real V = vk[cid];')
+                    o('  for (int p = p0_ + 4; p < p1_; ++p)')
+                    o('    b.ge[p] += (double)mu_ * (double)(V -'
+                      ' vk[a.nbr_idx[p]]);')
+                    o('}')
+            if meet_twice:
+                o('mkg_parts_sync();')
+            return out
+
+        body = []
+        for p in range(parts):
+            o = lambda x: body.append(tab + x)  # noqa: E731
+            o(f'{"if" if p == 0 else "else if"} (part_ == {p}) {{')
+            m = len(held[p])
+            for q, t in enumerate(held[p]):
+                o(f'    Real c{q} = __ldcg(tape + {t} * 32), n{q} = 0;')
+            for _, j, k in mine[p]:
+                if j is None:
+                    o(f'    Real f{k}_ = ((const Real *)b.gfield)'
+                      f'[(long long){k} * pitch + cid];')
+            last = p == parts - 1 and diff
+            edges = 0
+            if p == 0:
+                o('    const Real *lgrad = (const Real *)b.lgrad;')
+                o('    const int col_ = live ? b.probe_col[cid] : -1;')
+                o('    int row_ = a.steps[n - 1].log_row;')
+                o('    Real next_ = row_ >= 0 && col_ >= 0 ? lgrad['
+                  '(long long)row_ * b.nprobe + col_] : (Real)0;')
+                o('    row_ = n > 1 ? a.steps[n - 2].log_row : -1;')
+                if diff:
+                    o('    Real mu_ = ms[1][lane];')
+            if last:
+                o('    Real gx_ = ((const Real *)b.gg)[cid];')
+                o('    Real gy_ = ((const Real *)b.gg)[pitch + cid];')
+                edges = {_exp.DIFF_GRID: 0, _exp.DIFF_CONN: 4}.get(
+                    diff, extra)
+                where = [f'live ? b.ge[{q} * pitch + cid] : 0'
+                         for q in range(edges)]
+                if diff == _exp.DIFF_CONN:
+                    where = [f'p0_ + {q} < p1_ ? b.ge[p0_ + {q}] : 0'
+                             for q in range(4)]
+                for q in range(edges):
+                    o(f'    double e{q}_ = {where[q]};')
+            o('    for (int s = 0; s < n; ) {')
+            body.extend(step(p, 'c', 'n', 0))
+            o('        if (++s == n) break;')
+            o('        {')
+            body.extend(step(p, 'n', 'c', 1))
+            o('        }')
+            o('        ++s;')
+            o('    }')
+            for _, j, k in mine[p]:
+                if j is None:
+                    o(f'    if (live) ((Real *)b.gfield)[(long long){k} *'
+                      f' pitch + cid] = f{k}_;')
+            if last:
+                o('    if (live) {')
+                o('        ((Real *)b.gg)[cid] = gx_;')
+                o('        ((Real *)b.gg)[pitch + cid] = gy_;')
+                for q in range(edges):
+                    if diff == _exp.DIFF_CONN:
+                        o(f'        if (p0_ + {q} < p1_) b.ge[p0_ + {q}] ='
+                          f' e{q}_;')
+                    else:
+                        o(f'        b.ge[{q} * pitch + cid] = e{q}_;')
+                o('    }')
+            o('}')
+        subs = {
+            '@NSLOT@': str(self.slots),
+            '@PARTS@': str(parts),
+            '@X0@': str(x0),
+            '@MINB_ADJ@': str(tiles_per_sm),
+            '@FORWARD@': '\n'.join(self._forward_values(tab)),
+            '@PARTIALS@': '\n'.join(partials),
+            '@ROWS@': '\n'.join(rows),
+            '@SWEEP@': '\n'.join(body),
+        }
+        text = _exp._read('adjoint_map.cu.in')
+        for k, v in subs.items():
+            text = text.replace(k, v)
+        return self.fwd.source() + '\n' + text
+
     @staticmethod
     def _join(fsrc, text):
         """Appends the adjoint kernel (the template from its declaration
@@ -455,22 +799,43 @@ class TissueAdjoint(object):
         be = sim._get_backend(kernel)
         # Generated once per forward kernel (the forward kernel's key covers
         # the model version, precision, fields and launch shape)
-        akey = (kernel.key(), self.min_blocks, self.threads, self.guards)
+        akey = (kernel.key(), self.min_blocks, self.threads, self.guards,
+                self._tiles_per_sm(kernel))
         ak = self._generated.get(akey)
         if ak is None:
             ak = shared_kernel(
                 ('adjoint', sim.model_code(), sim._rl) + akey,
-                lambda: self._make(kernel))
+                lambda: self._make(kernel, akey[-1]))
             self._generated = {akey: ak}
         key = (id(be), akey, self.segment_steps)
         if self._attached != key:
             cubin = compile_kernel(ak)
-            be.check(be.lib.mkg_adj_attach(be.h, cubin, len(cubin),
-                                           self.segment_steps))
+            if ak.parts:
+                be.check(be.lib.mkg_adj_attach_map(
+                    be.h, cubin, len(cubin), self.segment_steps, ak.slots,
+                    ak.parts))
+            else:
+                be.check(be.lib.mkg_adj_attach(be.h, cubin, len(cubin),
+                                               self.segment_steps))
             self._attached = key
         return be
 
-    def _make(self, kernel):
+    def _tiles_per_sm(self, kernel):
+        """
+        Tiles on an SM where the reverse of a resident simulation goes by
+        tape and sweep (:meth:`AdjointKernel._generate_map`), 0 where the
+        general reverse kernel runs: with launch options of its own, and on
+        grids that fill the SMs with it.
+        """
+        sim = self.sim
+        if not kernel.team or sim._team is not None or self.guards or \
+                self.threads is not None or self.min_blocks != 1:
+            return 0
+        nx, ny = (sim._nx, sim._ny) if kernel.two_d else (sim._ntotal, 1)
+        n = -(-(-(-nx // 32) * ny) // autotune._sm_count(sim._device))
+        return n if n <= _MAP_TILES else 0
+
+    def _make(self, kernel, tiles_per_sm):
         """The adjoint kernel of a forward kernel."""
         sim = self.sim
         # The trajectory-writing forward kernel has the launch shape,
@@ -486,6 +851,10 @@ class TissueAdjoint(object):
             stage_lazy=kernel.stage_lazy, sync=kernel.sync,
             team=kernel.team)
         threads = self.threads
+        if tiles_per_sm:
+            ak = AdjointKernel(fwd, tiles_per_sm=tiles_per_sm)
+            if ak.parts:
+                return ak
         if threads is None and kernel.team:
             # A resident kernel's CTA is one tile; the reverse kernel's
             # warps each own tiles: as many warps as there are tiles for an

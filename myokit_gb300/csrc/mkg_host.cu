@@ -398,7 +398,11 @@ struct mkg_sim {
 
     /* Adjoint */
     cudaLibrary_t adj_lib = nullptr;
-    cudaKernel_t adj_fwd = nullptr, adj_bwd = nullptr;
+    cudaKernel_t adj_fwd = nullptr, adj_bwd = nullptr, adj_tape = nullptr;
+    void *d_tape = nullptr;               /* step matrices of a stretch */
+    long long tape_steps = 0;             /* its steps */
+    int adj_slots = 0;                    /* numbers per cell and step; 0:
+                                             the general reverse kernel */
     int adj_occ_fwd = 1, adj_occ_bwd = 1;
     int adj_bwd_threads = 0;              /* reverse kernel CTA size */
     size_t ckpt_bytes = 0;                /* bytes per checkpoint */
@@ -908,6 +912,7 @@ void mkg_destroy(mkg_sim *s)
     dfree(s->d_status);
     dfree(s->d_warp_epoch);
     dfree(s->d_vtag);
+    dfree(s->d_tape);
     dfree(s->d_stage);
     dfree(s->d_hi);
     dfree(s->d_hi_slot);
@@ -1932,8 +1937,18 @@ extern "C" int mkg_set_state_static(mkg_sim *s, const double *state,
 /* Discrete adjoint                                                         */
 /* ------------------------------------------------------------------------ */
 
-extern "C" int mkg_adj_attach(mkg_sim *s, const void *cubin, size_t size,
-                              int32_t seg_steps)
+namespace {
+
+/* Memory for the step matrices of a stretch of steps. Each stretch is two
+ * launches and the sweep's start: 96 x 96 cells, 48 states, 200 steps
+ * (7.8 MB each) 3.7 ms forward and backward with 64 MB, which stay in L2,
+ * 3.5 with 512 MB, 3.5 with 2 GB */
+const size_t kTapeBytes = (size_t)512 << 20;
+
+/* `slots` > 0: the tape and sweep kernels with that many numbers per cell
+ * and step and `parts` warps per tile, else the general reverse kernel */
+int adj_attach(mkg_sim *s, const void *cubin, size_t size,
+               int32_t seg_steps, int32_t slots, int32_t parts)
 {
     if (!s || !cubin || !size) return set_err(s, MKG_ERR_ARG, "null argument");
     if (seg_steps < 1) return set_err(s, MKG_ERR_ARG, "seg_steps < 1");
@@ -1945,7 +1960,12 @@ extern "C" int mkg_adj_attach(mkg_sim *s, const void *cubin, size_t size,
                               nullptr, nullptr, 0));
     CK(s, cudaLibraryGetKernel(&s->adj_fwd, s->adj_lib, "mkg_tissue_step"));
     CK(s, cudaLibraryGetKernel(&s->adj_bwd, s->adj_lib,
-                               "mkg_tissue_adjoint"));
+                               slots ? "mkg_adjoint_sweep"
+                                     : "mkg_tissue_adjoint"));
+    if (slots)
+        CK(s, cudaLibraryGetKernel(&s->adj_tape, s->adj_lib,
+                                   "mkg_adjoint_tape"));
+    s->adj_slots = slots;
     const int threads = s->cfg.block_x * s->cfg.block_y;
     /* The trajectory kernel stages tiles like the simulation's kernel */
     if (s->cfg.stage)
@@ -1960,10 +1980,18 @@ extern "C" int mkg_adj_attach(mkg_sim *s, const void *cubin, size_t size,
     s->adj_bwd_threads = fa.maxThreadsPerBlock;
     if (s->adj_bwd_threads < 32 || s->adj_bwd_threads % 32)
         return set_err(s, MKG_ERR_ARG, "invalid reverse kernel CTA size");
+    if (slots && s->adj_bwd_threads != parts * 32)
+        return set_err(s, MKG_ERR_ARG, "invalid sweep kernel CTA size");
     CK(s, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &s->adj_occ_bwd, (const void *)s->adj_bwd, s->adj_bwd_threads, 0));
     if (s->adj_occ_fwd < 1 || s->adj_occ_bwd < 1)
         return set_err(s, MKG_ERR_CUDA, "adjoint kernels cannot be resident");
+    mkg_launch geometry;
+    fill_launch(s, &geometry);
+    const long long tiles =
+        (long long)geometry.ntiles_x * geometry.ntiles_y;
+    if (slots && tiles > (long long)s->adj_occ_bwd * s->num_sms)
+        return set_err(s, MKG_ERR_CUDA, "adjoint tiles cannot be resident");
     {
         /* The trajectory kernel's grid may be larger than the forward's */
         const size_t nw = (size_t)s->adj_occ_fwd * s->num_sms *
@@ -1993,7 +2021,41 @@ extern "C" int mkg_adj_attach(mkg_sim *s, const void *cubin, size_t size,
     CK(s, cudaMalloc((void **)&s->d_fsteps, seg_steps * sizeof(mkg_step)));
     CK(s, cudaMalloc((void **)&s->d_bsteps, seg_steps * sizeof(mkg_step)));
     s->adj_seg = seg_steps;
+    dfree(s->d_tape);
+    s->tape_steps = 0;
+    if (slots) {
+        const size_t step = (size_t)tiles * slots * 32 * s->real;
+        long long n = std::min<long long>(
+            seg_steps, std::max<long long>(1, kTapeBytes / step));
+        /* (with less memory at hand shorter stretches) */
+        cudaError_t e;
+        while ((e = cudaMalloc(&s->d_tape, step * n)) ==
+                   cudaErrorMemoryAllocation && n > 1) {
+            cudaGetLastError();
+            s->d_tape = nullptr;
+            n /= 2;
+        }
+        CK(s, e);
+        s->tape_steps = n;
+    }
     return MKG_OK;
+}
+
+}  /* namespace */
+
+extern "C" int mkg_adj_attach(mkg_sim *s, const void *cubin, size_t size,
+                              int32_t seg_steps)
+{
+    return adj_attach(s, cubin, size, seg_steps, 0, 0);
+}
+
+extern "C" int mkg_adj_attach_map(mkg_sim *s, const void *cubin, size_t size,
+                                  int32_t seg_steps, int32_t slots,
+                                  int32_t parts)
+{
+    if (s && (slots < 1 || parts < 1 || parts > 32 || !s->cfg.team))
+        return set_err(s, MKG_ERR_ARG, "invalid adjoint tape");
+    return adj_attach(s, cubin, size, seg_steps, slots, parts);
 }
 
 extern "C" int mkg_adj_forward(mkg_sim *s, double tmin, double tmax,
@@ -2114,6 +2176,18 @@ int launch_coop(mkg_sim *s, cudaKernel_t k, void *arg, int occ,
     /* A staging kernel takes the tensor maps as a second parameter */
     void *args[] = {arg, &s->tmaps};
     CK(s, cudaLaunchKernelExC(&lc, (const void *)k, args));
+    s->n_launches++;
+    return MKG_OK;
+}
+
+int launch_plain(mkg_sim *s, cudaKernel_t k, void *arg, long long blocks,
+                 int threads)
+{
+    if (blocks > 0x7fffffff)
+        return set_err(s, MKG_ERR_ARG, "too many cells and steps");
+    void *args[] = {arg};
+    CK(s, cudaLaunchKernel((const void *)k, dim3((unsigned)blocks, 1, 1),
+                           dim3(threads, 1, 1), args, 0, s->stream));
     s->n_launches++;
     return MKG_OK;
 }
@@ -2253,6 +2327,35 @@ int adj_backward(mkg_sim *s, const double *lgrad, int64_t rows,
         b.lgrad = s->d_lgrad;
         b.nprobe = ncol;
         b.mu_sel = mu_sel;
+        if (s->adj_slots) {
+            /* Stretches of it, last first: their step matrices, then the
+             * steps. V's words now carry mu, the steps counted over the
+             * segment */
+            r = reset_step_words(s);
+            if (r) return r;
+            const long long tiles = (long long)a.ntiles_x * a.ntiles_y;
+            int epoch = 0;
+            for (long long hi = n; hi > 0;) {
+                const long long m = std::min(hi, s->tape_steps);
+                hi -= m;
+                b.f.steps = s->d_bsteps + st0 + hi;
+                b.f.nsteps = (int)m;
+                b.f.epoch_base = epoch;
+                b.traj = (const char *)s->d_traj +
+                         (size_t)hi * s->cfg.n_state * plane;
+                b.tape = s->d_tape;
+                b.mu_sel = mu_sel;
+                r = launch_plain(s, s->adj_tape, &b, (tiles * m + 3) / 4,
+                                 128);
+                if (r) return r;
+                r = launch_coop(s, s->adj_bwd, &b, s->adj_occ_bwd, tiles, 0,
+                                s->adj_bwd_threads);
+                if (r) return r;
+                epoch += (int)(m - 1);
+                mu_sel ^= (int)(m & 1);
+            }
+            continue;
+        }
         CK(s, cudaMemsetAsync(&s->d_status->barrier, 0, sizeof(unsigned),
                               s->stream));
         const long long bwd_blocks =

@@ -133,6 +133,8 @@ typedef struct mkg_adj_launch {
                                 double[4][pitch] (the edge to the left,
                                 right, down and up neighbour), connections
                                 double[n_nbr] (one per CSR entry) */
+    void *tape;              /* step matrices of a stretch of steps:
+                                Real[nsteps][tiles][slots][32] */
 } mkg_adj_launch;
 
 /* Accumulation modes for selected states of a single precision kernel */
