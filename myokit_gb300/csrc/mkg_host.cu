@@ -401,6 +401,8 @@ struct mkg_sim {
     cudaKernel_t adj_fwd = nullptr, adj_bwd = nullptr, adj_tape = nullptr;
     void *d_tape = nullptr;               /* step matrices of a stretch */
     long long tape_steps = 0;             /* its steps */
+    long long traj_segment = -1;          /* whose trajectory d_traj holds */
+    bool record = false;                  /* forward runs record it */
     int adj_slots = 0;                    /* numbers per cell and step; 0:
                                              the general reverse kernel */
     int adj_occ_fwd = 1, adj_occ_bwd = 1;
@@ -1137,6 +1139,7 @@ int mkg_get_state(mkg_sim *s, double *state, int64_t n)
 int mkg_set_fields(mkg_sim *s, const double *field_data, int64_t n)
 {
     if (!s) return set_err(s, MKG_ERR_ARG, "null argument");
+    s->traj_segment = -1;
     if (n != s->ncell * s->cfg.n_field)
         return set_err(s, MKG_ERR_ARG,
                        "field data must have nx * ny * n_field entries");
@@ -1152,6 +1155,7 @@ int mkg_set_fields(mkg_sim *s, const double *field_data, int64_t n)
 int mkg_set_conductance(mkg_sim *s, double gx, double gy)
 {
     if (!s) return set_err(s, MKG_ERR_ARG, "null argument");
+    s->traj_segment = -1;
     if (gx < 0) return set_err(s, MKG_ERR_ARG, "Invalid conductance gx=%g", gx);
     if (gy < 0) return set_err(s, MKG_ERR_ARG, "Invalid conductance gy=%g", gy);
     s->gx = gx;
@@ -1163,6 +1167,7 @@ int mkg_set_conductance_field(mkg_sim *s, const double *gx, int64_t ngx,
                               const double *gy, int64_t ngy)
 {
     if (!s) return set_err(s, MKG_ERR_ARG, "null argument");
+    s->traj_segment = -1;
     const long long nx = s->cfg.nx, ny = s->cfg.ny;
     if (ngx != ny * (nx - 1))
         return set_err(s, MKG_ERR_ARG, "gx must have ny * (nx - 1) entries");
@@ -1197,6 +1202,7 @@ int mkg_set_connections(mkg_sim *s, const int64_t *c1, const int64_t *c2,
                         const double *g, int64_t n)
 {
     if (!s) return set_err(s, MKG_ERR_ARG, "null argument");
+    s->traj_segment = -1;
     if (n < 0 || (n > 0 && (!c1 || !c2 || !g)))
         return set_err(s, MKG_ERR_ARG, "invalid connection arrays");
     const long long nc = s->ncell;
@@ -1248,6 +1254,7 @@ int mkg_set_connections(mkg_sim *s, const int64_t *c1, const int64_t *c2,
 int mkg_set_pacing_mode(mkg_sim *s, int32_t mode)
 {
     if (!s) return set_err(s, MKG_ERR_ARG, "null argument");
+    s->traj_segment = -1;
     if (mode < MKG_PACE_ALL || mode > MKG_PACE_NONE)
         return set_err(s, MKG_ERR_ARG, "invalid pacing mode");
     s->pace_mode = mode;
@@ -1258,6 +1265,7 @@ int mkg_set_paced_rect(mkg_sim *s, int64_t nx, int64_t ny, int64_t x,
                        int64_t y)
 {
     if (!s) return set_err(s, MKG_ERR_ARG, "null argument");
+    s->traj_segment = -1;
     s->px0 = x;
     s->px1 = x + nx;
     s->py0 = y;
@@ -1269,6 +1277,7 @@ int mkg_set_paced_rect(mkg_sim *s, int64_t nx, int64_t ny, int64_t x,
 int mkg_set_paced_list(mkg_sim *s, const int64_t *cells, int64_t n)
 {
     if (!s) return set_err(s, MKG_ERR_ARG, "null argument");
+    s->traj_segment = -1;
     const long long words = (s->ncell + 31) / 32;
     std::vector<unsigned int> bits(words, 0u);
     for (int64_t i = 0; i < n; ++i) {
@@ -1370,6 +1379,7 @@ int mkg_run_begin(mkg_sim *s, double tmin, double tmax, double default_dt,
                   double log_interval)
 {
     if (!s) return set_err(s, MKG_ERR_ARG, "null argument");
+    s->traj_segment = -1;
     if (!(default_dt > 0))
         return set_err(s, MKG_ERR_ARG, "Step size must be greater than zero.");
     if (!(log_interval > 0))
@@ -1545,7 +1555,7 @@ int mkg_run_chunk(mkg_sim *s, int64_t max_steps, double *t_out,
     const int64_t nlaunch = (n + spl - 1) / spl;
     /* (graphs are not used with a partner, whose log buffers may grow
      * between chunks) */
-    const bool graph = s->use_graphs && nlaunch > 1 && !p;
+    const bool graph = s->use_graphs && nlaunch > 1 && !p && !s->record;
     const int v_sel0 = s->v_sel;
     cudaGraphExec_t exec = nullptr;
     if (graph) {
@@ -1568,6 +1578,9 @@ int mkg_run_chunk(mkg_sim *s, int64_t max_steps, double *t_out,
             a.step0 = (int)off;
             a.epoch_base = epoch;
             a.v_sel = diffusion_on(s) ? (v_sel0 ^ (int)(off & 1)) : 0;
+            if (s->record)
+                a.traj = (char *)s->d_traj + (size_t)off * s->cfg.n_state *
+                                                 s->pitch * s->real;
             void *args[] = {&a, &s->tmaps};
             void *args_p[] = {&a, &b, &s->junction};
             cudaLaunchConfig_t lc;
@@ -1591,7 +1604,8 @@ int mkg_run_chunk(mkg_sim *s, int64_t max_steps, double *t_out,
             lc.gridDim = dim3((unsigned)grid, 1, 1);
             lc.dynamicSmemBytes = s->tile_smem;
             const cudaError_t e = cudaLaunchKernelExC(
-                &lc, (const void *)s->kernel, p ? args_p : args);
+                &lc, (const void *)(s->record ? s->adj_fwd : s->kernel),
+                p ? args_p : args);
             if (e != cudaSuccess) {
                 if (graph) {
                     cudaGraph_t g = nullptr;
@@ -2021,6 +2035,7 @@ int adj_attach(mkg_sim *s, const void *cubin, size_t size,
     CK(s, cudaMalloc((void **)&s->d_fsteps, seg_steps * sizeof(mkg_step)));
     CK(s, cudaMalloc((void **)&s->d_bsteps, seg_steps * sizeof(mkg_step)));
     s->adj_seg = seg_steps;
+    s->traj_segment = -1;
     dfree(s->d_tape);
     s->tape_steps = 0;
     if (slots) {
@@ -2082,6 +2097,11 @@ extern "C" int mkg_adj_forward(mkg_sim *s, double tmin, double tmax,
         s->ckpt_bytes = ckpt_bytes;
     }
     size_t nseg = 0;
+    mkg_launch geometry;
+    fill_launch(s, &geometry);
+    const bool record = s->cfg.team > 0 && !s->partner &&
+                        blocks_needed(s, &geometry) <=
+                            (long long)s->adj_occ_fwd * s->num_sms;
     int status = MKG_OK;
     while (status == MKG_OK) {
         /* Checkpoint: state planes, the current V plane and the
@@ -2102,9 +2122,16 @@ extern "C" int mkg_adj_forward(mkg_sim *s, double tmin, double tmax,
                                   s->d_hi, hi_bytes,
                                   cudaMemcpyDeviceToDevice, s->stream));
         s->adj_seg_vsel.push_back(s->v_sel);
+        /* A resident simulation's steps record their trajectory on the way:
+         * the backward pass starts with the last segment and need not
+         * recompute that one. us per step without and with the stores:
+         * 96 x 96 cells, 48 states 3.2, 3.7; 64 cells, 8 states, double
+         * precision 2.6, 2.6 (a step recomputed takes as much again) */
         double t = 0;
         int64_t rows = 0;
+        s->record = record;
         status = mkg_run_chunk(s, s->adj_seg, &t, &rows);
+        s->record = false;
         if (status < 0) return status;
         if (status == MKG_HALT_NAN)
             return set_err(s, MKG_ERR_ARG,
@@ -2120,6 +2147,7 @@ extern "C" int mkg_adj_forward(mkg_sim *s, double tmin, double tmax,
         s->adj_log.insert(s->adj_log.end(), s->h_log,
                           s->h_log + rows * s->log_ncol);
         s->adj_rows += rows;
+        if (record && done > 0) s->traj_segment = (long long)nseg;
         nseg++;
     }
     if (rows_out) *rows_out = s->adj_rows;
@@ -2279,21 +2307,7 @@ int adj_backward(mkg_sim *s, const double *lgrad, int64_t rows,
         const long long n = s->adj_seg_len[g];
         if (n == 0) continue;
         const long long st0 = s->adj_seg_start[g];
-        /* Restore the segment's checkpoint */
-        const char *ck = (const char *)s->adj_ckpt[g];
         const int vsel = s->adj_seg_vsel[g];
-        const size_t vplane = (size_t)s->pitch * s->vbytes;
-        CK(s, cudaMemcpyAsync(s->d_state, ck, plane * s->cfg.n_state,
-                              cudaMemcpyDeviceToDevice, s->stream));
-        CK(s, cudaMemcpyAsync((char *)s->d_vbuf + (size_t)vsel * vplane,
-                              ck + plane * s->cfg.n_state, vplane,
-                              cudaMemcpyDeviceToDevice, s->stream));
-        if (s->d_hi && s->cfg.n_hi > 0)
-            CK(s, cudaMemcpyAsync(s->d_hi,
-                                  ck + plane * s->cfg.n_state + vplane,
-                                  (size_t)s->pitch * 8 * s->cfg.n_hi,
-                                  cudaMemcpyDeviceToDevice, s->stream));
-        /* Forward over the segment, recording the trajectory */
         mkg_launch a;
         fill_launch(s, &a);
         a.n_log_items = 0;
@@ -2304,13 +2318,31 @@ int adj_backward(mkg_sim *s, const double *lgrad, int64_t rows,
         a.v_sel = vsel;
         a.traj = s->d_traj;
         if (s->cfg.stage) a.stage_tx = (int)s->lay.tx;
-        CK(s, cudaMemsetAsync(&s->d_status->barrier, 0, sizeof(unsigned),
-                              s->stream));
-        int r = reset_step_words(s);
-        if (r) return r;
-        r = launch_coop(s, s->adj_fwd, &a, s->adj_occ_fwd,
-                            blocks_needed(s, &a), s->tile_smem);
-        if (r) return r;
+        int r = MKG_OK;
+        if (s->traj_segment != g) {
+            /* Restore the segment's checkpoint */
+            const char *ck = (const char *)s->adj_ckpt[g];
+            const size_t vplane = (size_t)s->pitch * s->vbytes;
+            CK(s, cudaMemcpyAsync(s->d_state, ck, plane * s->cfg.n_state,
+                                  cudaMemcpyDeviceToDevice, s->stream));
+            CK(s, cudaMemcpyAsync((char *)s->d_vbuf + (size_t)vsel * vplane,
+                                  ck + plane * s->cfg.n_state, vplane,
+                                  cudaMemcpyDeviceToDevice, s->stream));
+            if (s->d_hi && s->cfg.n_hi > 0)
+                CK(s, cudaMemcpyAsync(s->d_hi,
+                                      ck + plane * s->cfg.n_state + vplane,
+                                      (size_t)s->pitch * 8 * s->cfg.n_hi,
+                                      cudaMemcpyDeviceToDevice, s->stream));
+            /* Forward over the segment, recording the trajectory */
+            CK(s, cudaMemsetAsync(&s->d_status->barrier, 0, sizeof(unsigned),
+                                  s->stream));
+            r = reset_step_words(s);
+            if (r) return r;
+            r = launch_coop(s, s->adj_fwd, &a, s->adj_occ_fwd,
+                                blocks_needed(s, &a), s->tile_smem);
+            if (r) return r;
+            s->traj_segment = g;
+        }
         /* The segment in reverse */
         mkg_adj_launch b;
         memset(&b, 0, sizeof(b));

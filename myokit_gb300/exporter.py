@@ -1279,6 +1279,8 @@ class TissueKernel(object):
                 new = f'n{i}_'
             if i == self.i_vm:
                 b.append(f'vs[lane] = {new};')
+                if self.traj:
+                    b.append(f'xs[{i}][lane] = (Real){new};')
                 b.append('if (k + 1 < nsteps && live)\n' + tab +
                          f'        mkg_word_store(vout_, cid, {new},'
                          ' now_ + 1u);')
@@ -1426,7 +1428,6 @@ class TissueKernel(object):
             '@TEAM@': str(self.team),
             '@NSLOT@': str(self.team_nslot),
             '@TRAJ@': '1' if self.traj else '0',
-            '@TRAJ_VALUE@': 'xs[i][lane]',
             '@DEVICE@': _read('mkg_device.h'),
             '@FIELD_LOADS@': '\n'.join(
                 f'        if (part_ == {k % self.team}) fs[{k}][lane] = '

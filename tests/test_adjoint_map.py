@@ -134,3 +134,23 @@ def test_equals_general_kernel(br77, decker, case, precision, kw):
             far = np.max(np.abs(np.subtract(got, want)), initial=0)
             most = np.max(np.abs(want), initial=0)
             assert far <= (1e-11 if precision == DP else 1e-3) * most, k
+
+
+@pytest.mark.gpu
+def test_recorded_trajectory_is_recomputed_after_changes(br77):
+    # The forward run leaves the last segment's trajectory for the backward
+    # pass. Fields that a run changed in between apply to the backward pass,
+    # with the general kernel and with this one
+    out = []
+    for general in (True, False):
+        adj = _adjoint(br77, DP, 70, False, general, fields=['isi.gsBar'],
+                       probes=[0, 69], segment=200)
+        v = adj.forward(1.0, 0.13)
+        w = np.cos(np.arange(v.size)).reshape(v.shape)
+        before = adj.backward(w)['isi.gsBar']
+        adj.sim.set_field('isi.gsBar', np.linspace(0.05, 0.12, 70))
+        adj.sim.run(0.05)
+        out.append((before, adj.backward(w)['isi.gsBar']))
+    for a, b in zip(*out):
+        assert np.max(np.abs(a - b)) <= 1e-11 * np.max(np.abs(a))
+    assert not np.array_equal(*out[0]) and not np.array_equal(*out[1])
