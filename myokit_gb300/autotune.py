@@ -105,15 +105,15 @@ def resident_shape(tiles, sms, single):
     code an SM has to fetch. Measured, us per step with 1 / 2 / 4 / 8 warps
     per tile and (last) the undivided kernel, by tiles on an SM:
 
-    - 48 states, single precision: one tile 3.0 / 2.0 / 1.7 / 1.7, 5.3;
-      four 3.0 / 2.3 / 1.9 / 2.9, 5.3; six 3.4 / 2.4 / 2.5, 5.3; eight
+    - 48 states, single precision: one tile 3.0 / 2.3 / 1.7 / 1.7, 5.3;
+      four 3.0 / 2.2 / 1.9 / 2.8, 5.3; six 3.4 / 2.4 / 2.5, 5.3; eight
       3.5 / 2.9 / 3.3, 5.5; twelve 4.1 / 4.5, 7.2; sixteen 5.5 / 6.7, 7.4;
-    - the same in double precision: one tile 73 / 37 / 21 / 15, 83; two
-      73 / 37 / 23 / 30, 84; three 73 / 41 / 33 / 49, 83; four 74 / 41 / 49,
-      85; six 79 / 56 / 73, 84; eight 81 / 78, 95;
-    - 8 states, single precision: one 0.96 / 0.89 / 0.89 / 0.90, 2.3; eight
-      1.05 / 0.89 / 1.00, 2.4; sixteen 1.3 / 2.0, 3.0; double precision: one
-      11.1 / 6.6 / 6.2 / 6.0, 13.4; three 11.1 / 9.6 / 6.3 / 6.7, 13.4; six
+    - the same in double precision: one tile 73 / 36 / 21 / 15, 83; two
+      73 / 36 / 23 / 51, 84; three 73 / 40 / 35 / 44, 84; four 74 / 41 / 51,
+      85; six 79 / 57 / 74, 85; eight 81 / 77, 95;
+    - 8 states, single precision: one 0.94 / 0.85 / 0.87 / 0.90, 2.3; eight
+      1.05 / 0.88 / 1.00, 2.4; sixteen 1.3 / 2.0, 3.0; double precision: one
+      11.1 / 6.9 / 6.1 / 6.1, 13.4; three 11.1 / 9.6 / 6.2 / 7.0, 13.4; six
       15.8 / 11.0 / 10.4, 16.3; eight 13.3 / 12.0 / 15.6, 16.5.
 
     Nine tiles on an SM in double precision take 100 us with the 48 states,

@@ -1228,7 +1228,11 @@ class TissueKernel(object):
         team = _teams.Team(
             self.team, [(n, r, c) for n, r, _, c in items], gates,
             derivatives, first, _IDIFF,
-            _teams._COST[self.single]['rl'])
+            _teams._COST[self.single]['rl'],
+            _teams._HALO['double' if not self.single else
+                         'mixed' if self.v_double else 'single']
+            if self.diffusion != DIFF_NONE else 0,
+            _teams._TRIP[self.single], self.min_blocks <= 2)
         self.team_plan = team
         self.team_nslot = len(team.slots)
         halo = [p for p in range(self.team) if team.halo[p] or p == 0] \
@@ -1316,18 +1320,22 @@ class TissueKernel(object):
 
         # When the neighbours' V is asked for: its words are there about 500
         # cycles into a step, and a word asked for before that is asked for
-        # again where it is needed, a trip to L2 of 880 cycles; one asked for
-        # at the first meeting may not be back yet. So at the start of a step
-        # whose first phase is shorter than that trip (an addition counts as
-        # 5 cycles in single precision, 67 in double), and at the end of a
-        # longer one, which the wait is then hidden behind. us per step asked
-        # for at the start, before and after the first meeting: 48 states,
-        # 61 x 47 cells (1740 cycles) 1.64, 1.57, 1.61, 128 x 128 2.00, 1.91,
-        # 1.91; 8 states, 200 cells (390 cycles) 0.55, 0.60, 0.62, double
-        # precision (3500) 2.59, 2.58, 2.80.
+        # again where it is needed, a trip to L2 of 880 cycles.
+        # - A first phase longer than the trip and the current together: asked
+        #   for half a trip into it, the current taken at its end, by a warp
+        #   that has so much less to do there. With up to two tiles on an SM:
+        #   there a step is one tile's chain of latencies; with more the
+        #   other tiles' warps run meanwhile. us per step with the current in
+        #   the last phase and in the first: 48 states, 61 x 47 cells 1.57,
+        #   1.50; 128 x 70 (two tiles) 1.63, 1.55; 128 x 110 (three) 1.73,
+        #   1.86; 8 states, double precision, 200 cells 2.57, 2.35; 64 x 200
+        #   (three) 6.5, 7.6.
+        # - A first phase longer than the trip: asked for at its end (61 x 47
+        #   cells: at the start 1.64, so 1.57).
+        # - A shorter one: asked for at the start of the step (8 states,
+        #   single precision, 200 cells: 0.55; at the first meeting 0.60).
         nphase = len(team.work)
-        ask_late = nphase > 1 and \
-            max(team.cost[0]) > 880 / (5 if self.single else 67)
+        price_ = {n: c for n, _, _, c in items}
         out = []
         for p in range(self.team):
             gate_list = [i for f in range(nphase) for i in team.gates_of[f][p]]
@@ -1351,7 +1359,8 @@ class TissueKernel(object):
                 take = [f'{tab}    const Real {_IDIFF} = 0;',
                         f'{tab}    (void){_IDIFF};']
             early = p in halo and team.halo_early[p]
-            if p in halo and (early or not ask_late):
+            soon = team.halo_first and p in halo and not early
+            if p in halo and (early or not (soon or team.halo_late)):
                 out.append(f'{tab}    MKG_HALO_ASK()')
             if early:
                 out.extend(take)
@@ -1359,7 +1368,7 @@ class TissueKernel(object):
                 # Logged values, before any state changes; a NaN halt
                 out.append(f'{tab}    if (row >= 0) {{')
                 if not early:
-                    if halo and ask_late:
+                    if halo and (soon or team.halo_late):
                         out.append(f'{tab}    MKG_HALO_ASK()')
                     out.extend(take)
                 out.append(f'{tab}    if (live) {{')
@@ -1370,7 +1379,7 @@ class TissueKernel(object):
                 out.append(f'{tab}    MKG_CHECK_HALT()')
             after = []           # stores that wait for the team's loads
             for f in range(nphase):
-                if f == 1 and p in halo and ask_late and not early:
+                if f == 1 and p in halo and team.halo_late and not early:
                     out.append(f'{tab}    MKG_HALO_ASK()')
                 if f:
                     out.append(f'{tab}    mkg_team_sync();')
@@ -1381,13 +1390,21 @@ class TissueKernel(object):
                 for x in team.read[f][p]:
                     out.append(f'{tab}    const Real {x} = '
                                f'hs[{team.slots[x]}][lane];')
-                late = f == nphase - 1 and not early and (
+                late = f == nphase - 1 and not early and not soon and (
                     team.halo[p] or p == 0)
+                ask = soon and f == 0
+                spent = 0
                 for x in team.work[f][p]:
                     if late and _IDIFF in refs[x]:
                         out.extend(take)
                         late = False
+                    if ask and spent >= _teams._TRIP[self.single] / 2:
+                        out.append(f'{tab}    MKG_HALO_ASK()')
+                        ask = False
                     out.append(line_of[x])
+                    spent += price_[x]
+                if ask:
+                    out.append(f'{tab}    MKG_HALO_ASK()')
                 if late:
                     out.extend(take)
                 for x in team.written[f][p]:
@@ -1396,6 +1413,8 @@ class TissueKernel(object):
                     a, b = update(i)
                     out.extend(f'{tab}    {x}' for x in a)
                     (out if f else after).extend(f'{tab}    {x}' for x in b)
+                if soon and f == 0:
+                    out.extend(take)
             if nphase == 1:
                 # (a team of one warp: nothing changes hands)
                 out.append(f'{tab}    mkg_team_sync();')

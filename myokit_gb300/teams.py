@@ -34,8 +34,13 @@ CUBIC = 55
 _CHEAP = 1
 _AGAIN = 2.0
 _SHARE = 32
-# What the exchange of V adds to the warp that updates it
-_HALO = 40
+# What the diffusion current adds to the warp that updates V (in single
+# precision; with V in double precision there; in double precision)
+_HALO = {'single': 22, 'mixed': 240, 'double': 18}
+# What the wait and the current add to it in a last phase
+_LATER = 40
+# A trip to L2, 880 cycles, and what an addition counts as
+_TRIP = {True: 880 / 5, False: 880 / 67}
 
 
 def cost(e, single):
@@ -94,9 +99,13 @@ class Team(object):
     phase. Between phases the team meets; ``slots`` maps the names handed
     over to their slots, ``written[f][w]`` and ``read[f][w]`` list those a
     warp writes at the end and reads at the start of a phase. ``cost[f][w]``
-    is the estimated time.
+    is the estimated time. ``exchange`` is what the diffusion current adds to
+    the first warp, in the first phase (``halo_first``, if ``soon``) where
+    there is time for it and a ``trip`` for the words, else in the last (``halo_late``: the
+    first phase has time for the trip).
     """
-    def __init__(self, n, items, gates, derivatives, first, halo, rl_cost):
+    def __init__(self, n, items, gates, derivatives, first, halo, rl_cost,
+                 exchange=0, trip=0, soon=True):
         self.n = n
         order = [name for name, _, _ in items]
         refs = {name: r for name, r, _ in items}
@@ -140,6 +149,7 @@ class Team(object):
             self.cost = [[total(needed)]]
             self.halo = [bool(needs_halo & needed)]
             self.halo_early = [False]
+            self.halo_first = self.halo_late = False
             return
 
         # What several equations need and is dear enough to be computed once,
@@ -201,8 +211,18 @@ class Team(object):
             return sorted(us, key=lambda u: (-(total(u[1]) + u[2]),
                                              str(u[0])))
         none = [0.0] * n
+        # The current is taken in the first phase, by a warp that has so much
+        # less to do there, where the words are back before that phase ends
+        opening = (total(closure(shared)) if shared else sum(
+            total(u[1]) + u[2] for u in units)) / n
+        self.halo_first = soon and first is not None and exchange > 0 and \
+            opening > trip + exchange
+        self.halo_late = not self.halo_first and opening > trip
+        begin = exchange if self.halo_first else 0
+        later = 0 if self.halo_first else _LATER
         if shared:
             phase()
+            self.cost[0][0] += begin
             for u in largest_first([(('value', x), closure([x]), 1)
                                     for x in order if x in shared]):
                 place(*u, none)
@@ -225,9 +245,11 @@ class Team(object):
             own = closure([d], [x for x in refs if x not in tail])
             tails[i] = own
         phase()
+        if not shared:
+            self.cost[0][0] += begin
         bias = list(none)
         if first is not None:
-            bias[0] = _HALO
+            bias[0] = later
         for u in largest_first(units):
             place(*u, bias)
         if shared:
@@ -257,7 +279,7 @@ class Team(object):
             return (total(tails[i] - groups[last][w]) + 2 +
                     2 * len(inputs(i) - have))
         if first is not None:
-            self.cost[last][0] += spend(first, 0) + _HALO
+            self.cost[last][0] += spend(first, 0) + later
             groups[last][0] |= tails[first]
             self.tails_of[0].append(first)
         for i in sorted((i for i in derivatives if i != first),

@@ -112,23 +112,28 @@ def test_equations_that_are_alike(decker, team):
 
 
 def test_when_neighbours_are_asked(decker, br77):
-    # At the start of a step whose first phase is short, at the end of a
-    # long first phase, and where one warp does all at the start
-    for m, rl, precision, team, late in (
+    # In a long first phase the words are asked for on the way and the
+    # current is taken before the team meets; else they are asked for at the
+    # start of a step and the current is taken in the last phase
+    for m, rl, precision, team, soon in (
             (decker, True, SP, 4, True), (decker, True, SP, 1, False),
-            (br77, False, SP, 4, False), (br77, False, DP, 8, True)):
-        body = _kernel(m, precision, team, rl).team_body
-        first = body.index('const Real', body.index('part_ == 0'))
-        asks = [i for i in range(len(body))
-                if body.startswith('MKG_HALO_ASK()', i)]
-        meets = body.index('mkg_team_sync();')
-        log = body.index('if (row >= 0)')
-        assert asks and first < asks[0]
-        if late:
-            assert log < asks[0] and asks[-1] > asks[0]
-            assert body[asks[1]:meets].count('\n') == 1
+            (br77, False, SP, 4, False), (br77, False, DP, 8, True),
+            (decker, True, SP, 16, False), (decker, True, DP, 16, True)):
+        k = _kernel(m, precision, team, rl)
+        assert k.team_plan.halo_first == soon
+        body = k.team_body
+        body = body[:body.index('else if (part_') if team > 1 else None]
+        # (after the log row's own copy)
+        rest = body[body.index('MKG_CHECK_HALT'):]
+        meets = rest.index('mkg_team_sync();')
+        assert rest.count('MKG_HALO(id_)') == 1
+        assert rest.count('MKG_HALO_ASK()') == int(soon)
+        if soon:
+            assert rest.index('MKG_HALO_ASK()') < \
+                rest.index('MKG_HALO(id_)') < meets
         else:
-            assert asks[0] < log
+            assert body.index('MKG_HALO_ASK()') < body.index('row >= 0')
+            assert team == 1 or rest.index('MKG_HALO(id_)') > meets
 
 
 @pytest.mark.parametrize('precision', [SP, DP])
