@@ -127,7 +127,7 @@ def resident_shape(tiles, sms, single):
     return None
 
 
-def default_shape(single, n_state, plane_bytes):
+def default_shape(single, n_state, plane_bytes, tiles_per_sm):
     """
     The launch shape of a grid too large for resident tiles, where nobody
     chose one: ``(threads, CTAs per SM, lazy staging, synchronisation)``.
@@ -141,8 +141,15 @@ def default_shape(single, n_state, plane_bytes):
       and 101; 8 states 2048 x 2048 74 and 74. The many tiles of a warp
       even out what neighbours wait for, and no warp idles at a barrier
       while memory does;
-    - planes within it: 256 x 2 with the barrier (512 x 512, 48 states: 20.7
-      against 20.3, 300 x 400 per-edge 13.1 and 13.4, 8 states 6.3 and 6.9);
+    - many states, 60 tiles per SM and more, planes in the L2: the same (48
+      states, 640 x 520 25.8 against 27.8, Kahan 28.5 and 29.7, per-edge
+      Kahan 32.3 and 32.9, FP64 accumulation 54.6 and 54.6; 800 x 700 41.6
+      and 44.6, Kahan 46.8 and 54.2);
+    - else 256 x 2 with the barrier (512 x 512, 54 tiles per SM, 20.9
+      against 20.7, Kahan 22.4 and 22.6, per-edge 23.1 and 23.9, FP64
+      accumulation 41.4 and 43.0; 8 states 640 x 520 8.0 and 8.2, 512 x 512
+      6.4 and 7.1, 290 x 290 4.0 and 4.7: their steps are too short to hide
+      the neighbours' counters);
     - double precision, many states: 8 warps per SM of 64-thread CTAs, read
       from shared memory where used: 256 x 256 114 against 180 with 128
       threads and prefetch, 301 x 211 119 and 182, 512 x 512 491 and 676;
@@ -152,7 +159,7 @@ def default_shape(single, n_state, plane_bytes):
     if not single:
         return (64, 4, 1, 'barrier') if n_state >= 16 else (
             512, 1, 1, 'barrier')
-    if plane_bytes > 120e6:
+    if plane_bytes > 120e6 or (tiles_per_sm >= 60 and n_state >= 16):
         return 512, 1, 0, 'neighbors'
     return 256, 2, 0, 'barrier'
 

@@ -817,8 +817,11 @@ class SimulationCUDA(object):
         planes = self._nstate * (4 if single else 8)
         if self._accumulate:
             planes += 4 * len(self.accumulated_states())
-        return autotune.default_shape(single, self._nstate,
-                                      planes * self._ntotal)
+        tiles = -(-self._nx // 32) * self._ny if len(self._dims) == 2 \
+            else -(-self._ntotal // 32)
+        return autotune.default_shape(
+            single, self._nstate, planes * self._ntotal,
+            tiles / autotune._sm_count(self._device))
 
     def _sync_mode(self):
         """How steps are separated: 'barrier' or 'neighbors'."""

@@ -175,6 +175,18 @@ def test_launch_shape_of_large_grids(decker, br77):
             96, 1, 0, 'barrier')
 
 
+def test_launch_shape_between_resident_and_memory_bound(decker, br77):
+    # 60 tiles per SM: many rounds of tiles per warp, planes still in L2
+    for m, rl, n, want in (
+            (decker, True, (640, 457), (512, 1, 0, 'neighbors')),
+            (decker, True, (640, 455), (256, 2, 0, 'barrier')),
+            (decker, True, 292000, (512, 1, 0, 'neighbors')),
+            (br77, False, (640, 457), (256, 2, 0, 'barrier'))):
+        k = mg.SimulationCUDA(m, None, ncells=n, precision=SP,
+                              rl=rl)._kernel([])
+        assert (k.block[0], k.min_blocks, k.stage_lazy, k.sync) == want
+
+
 def test_large_models_and_launch_options_are_not_resident(br77):
     s = mg.SimulationCUDA(br77, None, ncells=64)
     assert s._kernel([]).team == 4
