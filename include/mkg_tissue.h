@@ -297,6 +297,11 @@ int mkg_last_stats(const mkg_sim *sim, double *kernel_ms, int64_t *launches,
  */
 int mkg_adj_attach(mkg_sim *sim, const void *cubin, size_t size,
                    int32_t seg_steps);
+/* The same for a resident simulation's module with mkg_adjoint_tape and
+ * mkg_adjoint_sweep instead of the reverse kernel: `slots` numbers per cell
+ * and step, `parts` warps per tile of the sweep. */
+int mkg_adj_attach_map(mkg_sim *sim, const void *cubin, size_t size,
+                       int32_t seg_steps, int32_t slots, int32_t parts);
 int mkg_adj_forward(mkg_sim *sim, double tmin, double tmax, double dt,
                     double log_interval, int64_t *rows);
 int mkg_adj_read_log(mkg_sim *sim, double *values, int64_t rows);
