@@ -17,9 +17,11 @@ exact gradients of what the forward kernel computes, up to rounding.
 - :class:`AdjointKernel` emits, from the forward :class:`TissueKernel`'s
   equation list, a CUDA kernel that re-evaluates the model at step k from a
   recorded trajectory and sweeps the equations in reverse.
+  For small grids two kernels instead: the sparse matrix of every cell and
+  step at once, and a sweep that multiplies through them.
 - :class:`TissueAdjoint` runs forward with checkpoints every K steps, then
   per segment (last first) recomputes the trajectory and runs the adjoint
-  kernel; :class:`TissueLossFunction` wraps this as a
+  kernels; :class:`TissueLossFunction` wraps this as a
   ``torch.autograd.Function``.
 """
 import math
