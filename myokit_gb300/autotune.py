@@ -95,7 +95,7 @@ def lookup(sim):
     return None
 
 
-def resident_shape(tiles, sms, single):
+def resident_shape(tiles, sms, single, n_state=16):
     """
     ``(warps per tile, CTAs per SM)`` of a resident kernel
     (``csrc/resident_kernel.cu.in``) for a grid of ``tiles`` warp tiles, or
@@ -112,15 +112,18 @@ def resident_shape(tiles, sms, single):
       73 / 36 / 23 / 51, 84; three 73 / 40 / 35 / 44, 84; four 74 / 41 / 51,
       85; six 79 / 57 / 74, 85; eight 81 / 77, 95;
     - 8 states, single precision: one 0.94 / 0.85 / 0.87 / 0.90, 2.3; eight
-      1.05 / 0.88 / 1.00, 2.4; sixteen 1.3 / 2.0, 3.0; double precision: one
-      11.1 / 6.9 / 6.1 / 6.1, 13.4; three 11.1 / 9.6 / 6.2 / 7.0, 13.4; six
-      15.8 / 11.0 / 10.4, 16.3; eight 13.3 / 12.0 / 15.6, 16.5.
+      1.05 / 0.88 / 1.00, 2.4; sixteen 1.3 / 2.0, 3.0;
+    - the same in double precision: one 12.2 / 6.9 / 4.1 / 2.8, 13.4; two
+      12.2 / 6.9 / 4.5 / 3.4, 13.4; four 12.5 / 8.4 / 6.3 / 5.7, 13.6; five
+      13.6 / 8.9 / 7.0, 16.3; eight 14.3 / 11.2 / 10.6, 16.5. Its code is
+      small enough for many warps (fewer than 16 states).
 
     Nine tiles on an SM in double precision take 100 us with the 48 states,
     the undivided kernel 94: its 8 warps per SM have the registers they need.
     """
     per = -(-tiles // sms)
     for team, most in ((4, 4), (2, 8), (1, 16)) if single else (
+            (8, 4), (4, 8)) if n_state < 16 else (
             (8, 1), (4, 3), (2, 7), (1, 8)):
         if per <= most:
             return team, per
@@ -216,7 +219,8 @@ def _resident_candidates(sim):
     two_d = len(sim._dims) == 2 and sim._diffusion_mode() in (1, 2)
     nx, ny = (sim._nx, sim._ny) if two_d else (sim._ntotal, 1)
     shape = resident_shape(-(-nx // 32) * ny, _sm_count(sim._device),
-                           sim._precision == myokit.SINGLE_PRECISION)
+                           sim._precision == myokit.SINGLE_PRECISION,
+                           sim._nstate)
     if shape is None:
         return []
     team, minb = shape

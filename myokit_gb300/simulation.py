@@ -959,7 +959,7 @@ class SimulationCUDA(object):
             return int(hit['team']), int(hit['min_blocks'])
         return autotune.resident_shape(
             tiles, autotune._sm_count(self._device),
-            self._precision == myokit.SINGLE_PRECISION)
+            self._precision == myokit.SINGLE_PRECISION, self._nstate)
 
     def _kernel(self, inter_log):
         """The generated kernel for the current configuration (cached)."""

@@ -153,6 +153,19 @@ def test_shape_by_size():
         assert shape(152 * most + 1, 152, single) is None
 
 
+def test_shape_of_small_models(br77, decker):
+    # Fewer than 16 states in double precision: code for many warps
+    for tiles, want in ((7, (8, 1)), (152 * 4, (8, 4)), (152 * 4 + 1, (4, 5)),
+                        (152 * 8, (4, 8)), (152 * 8 + 1, None)):
+        assert autotune.resident_shape(tiles, 152, False, 8) == want
+        k = mg.SimulationCUDA(br77, None, ncells=32 * tiles,
+                              precision=DP)._kernel([])
+        assert k.team == (want[0] if want else 0)
+    k = mg.SimulationCUDA(decker, None, ncells=32 * 500, precision=DP,
+                          rl=True)._kernel([])
+    assert k.team == 2
+
+
 def test_launch_shape_of_large_grids(decker, br77):
     for m, rl, precision, n, kw, want in (
             (decker, True, SP, (512, 512), {}, (256, 2, 0, 'barrier')),
