@@ -113,9 +113,9 @@ def resident_shape(tiles, sms, single, n_state=16):
       85; six 79 / 57 / 74, 85; eight 81 / 77, 95;
     - 8 states, single precision: one 0.94 / 0.85 / 0.87 / 0.90, 2.3; eight
       1.05 / 0.88 / 1.00, 2.4; sixteen 1.3 / 2.0, 3.0;
-    - the same in double precision: one 12.2 / 6.9 / 4.1 / 2.8, 13.4; two
-      12.2 / 6.9 / 4.5 / 3.4, 13.4; four 12.5 / 8.4 / 6.3 / 5.7, 13.6; five
-      13.6 / 8.9 / 7.0, 16.3; eight 14.3 / 11.2 / 10.6, 16.5. Its code is
+    - the same in double precision: one 12.2 / 6.9 / 4.1 / 2.7, 13.4; two
+      12.2 / 6.9 / 4.5 / 3.2, 13.4; four 12.5 / 8.4 / 6.3 / 5.3, 13.6; five
+      13.6 / 8.9 / 7.0, 16.3; eight 14.3 / 11.2 / 10.3, 16.5. Its code is
       small enough for many warps (fewer than 16 states).
 
     Nine tiles on an SM in double precision take 100 us with the 48 states,

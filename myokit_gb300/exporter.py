@@ -1232,7 +1232,8 @@ class TissueKernel(object):
             _teams._HALO['double' if not self.single else
                          'mixed' if self.v_double else 'single']
             if self.diffusion != DIFF_NONE else 0,
-            _teams._TRIP[self.single], self.min_blocks <= 2)
+            _teams._TRIP[self.single], self.min_blocks <= 2 or
+            (not self.single and self.n_state < 16))
         self.team_plan = team
         self.team_nslot = len(team.slots)
         halo = [p for p in range(self.team) if team.halo[p] or p == 0] \
@@ -1327,9 +1328,11 @@ class TissueKernel(object):
         #   there a step is one tile's chain of latencies; with more the
         #   other tiles' warps run meanwhile. us per step with the current in
         #   the last phase and in the first: 48 states, 61 x 47 cells 1.57,
-        #   1.50; 128 x 70 (two tiles) 1.63, 1.55; 128 x 110 (three) 1.73,
-        #   1.86; 8 states, double precision, 200 cells 2.57, 2.35; 64 x 200
-        #   (three) 6.5, 7.6.
+        #   1.50; 128 x 70 (two tiles) 1.63, 1.55; 200 x 150 (seven) 2.84,
+        #   2.98; double precision, 64 x 500 (seven) 69, 82. Small models in
+        #   double precision are bound by their chains with more tiles, too:
+        #   8 states, 200 cells 2.70, 2.52; 64 x 300 (four) 5.56, 5.31; 64 x
+        #   600 (eight) 10.5, 10.3.
         # - A first phase longer than the trip: asked for at its end (61 x 47
         #   cells: at the start 1.64, so 1.57).
         # - A shorter one: asked for at the start of the step (8 states,

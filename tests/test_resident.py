@@ -161,6 +161,7 @@ def test_shape_of_small_models(br77, decker):
         k = mg.SimulationCUDA(br77, None, ncells=32 * tiles,
                               precision=DP)._kernel([])
         assert k.team == (want[0] if want else 0)
+        assert not want or k.team_plan.halo_first
     k = mg.SimulationCUDA(decker, None, ncells=32 * 500, precision=DP,
                           rl=True)._kernel([])
     assert k.team == 2
