@@ -284,7 +284,13 @@ class Team(object):
             self.tails_of[0].append(first)
         for i in sorted((i for i in derivatives if i != first),
                         key=lambda i: (-total(tails[i]), i)):
-            w = min(range(n), key=lambda w: (
+            # In the last phase the first warp stores V and publishes its
+            # word as soon as it has them, so where the current is taken
+            # there no other warp may: it would read V of the next step, or
+            # wait for words that a neighbour has overwritten meanwhile
+            alone = first is not None and exchange > 0 and \
+                not self.halo_first and tails[i] & needs_halo
+            w = 0 if alone else min(range(n), key=lambda w: (
                 self.cost[last][w] + spend(i, w), w))
             self.cost[last][w] += spend(i, w)
             groups[last][w] |= tails[i]
