@@ -1387,7 +1387,8 @@ class TissueKernel(object):
                 if f:
                     out.append(f'{tab}    mkg_team_sync();')
                 if f == 1:
-                    out.append(f'{tab}    if (s_stop) break;')
+                    out.append(f'{tab}    if (s_stop[stop_]) break;')
+                    out.append(f'{tab}    stop_ ^= 1;')
                     out.extend(after)
                     after = []
                 for x in team.read[f][p]:
@@ -1421,7 +1422,7 @@ class TissueKernel(object):
             if nphase == 1:
                 # (a team of one warp: nothing changes hands)
                 out.append(f'{tab}    mkg_team_sync();')
-                out.append(f'{tab}    if (s_stop) break;')
+                out.append(f'{tab}    if (s_stop[stop_]) break;')
                 out.extend(after)
             for i in team.tails_of[p]:
                 for x in sum(update(i), []):

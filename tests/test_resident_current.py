@@ -82,6 +82,40 @@ def test_current_of_default_launch_shapes(decker, br77):
                     _check_current(k)
 
 
+def _check_stop(k):
+    """A word that says to leave is not set in an interval between two
+    meetings in which another warp tests it: that warp could leave a step
+    before the others, which would wait for it at the next meeting. (Words
+    by the step's parity: 0 is the step's, 1 the next step's.)"""
+    sets, tests = {}, {}
+    for w, p in enumerate(_parts(k)):
+        word = 0
+        for f, x in enumerate(p):
+            for t in re.findall(r'MKG_HALO\(id_\)|MKG_CHECK_HALT\(\)|'
+                                r'if \(s_stop|stop_ \^= 1', x):
+                if t.startswith('stop_'):
+                    word ^= 1
+                else:
+                    (tests if t.startswith('if') else sets).setdefault(
+                        (f, word), set()).add(w)
+    assert set(tests) == {(1, 0)} and len(tests[1, 0]) == k.team
+    assert not set(sets) & set(tests)
+    # What is set before the test is tested in this step, else in the next
+    assert all(word == min(f, 1) for f, word in sets)
+    loop = k.source().split('for (; k < nsteps; ++k) {')[1]
+    assert set(re.findall(r's_stop\W?\w*\W?', loop)) == {'s_stop[stop_]'}
+    assert 'int stop_ = k & 1;' in loop
+
+
+@pytest.mark.parametrize('precision', [SP, DP])
+@pytest.mark.parametrize('team', [1, 2, 4, 8])
+def test_stop_word_is_not_tested_while_it_may_be_set(decker, br77, team,
+                                                     precision):
+    for m, rl, n in ((br77, False, 0), (br77, False, 2), (br77, True, 0),
+                     (decker, True, 0), (decker, True, 1)):
+        _check_stop(_kernel(_balances(m, n), precision, team, rl))
+
+
 # ---------------------------------------------------------------------------
 # GPU
 # ---------------------------------------------------------------------------
