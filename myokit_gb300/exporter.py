@@ -135,7 +135,7 @@ class CudaExpressionWriter(CBasedExpressionWriter):
     (``myokit/formats/opencl/_ewriter.py:59-93``).
     """
     def __init__(self, single, native_math=False, fast_divide=False,
-                 soft=False, fuse=False):
+                 soft=False, fuse=False, scale=True):
         super().__init__()
         self._single = bool(single)
         self._native = bool(native_math) and self._single
@@ -143,9 +143,10 @@ class CudaExpressionWriter(CBasedExpressionWriter):
         # Double precision exp and division in integer arithmetic
         # (csrc/mkg_math64.h)
         self._soft = bool(soft) and not self._single
-        # Multiply-adds and the scaling of single precision exponentials
-        # written out (see ex)
+        # Multiply-adds and (scale) the scaling of single precision
+        # exponentials written out (see ex)
         self._fuse = bool(fuse)
+        self._scale = bool(scale) and self._single and not self._native
         self.int_powers = set()
 
     # Kernels are compiled without the compiler's own contraction of
@@ -158,8 +159,7 @@ class CudaExpressionWriter(CBasedExpressionWriter):
         if self._fuse:
             if isinstance(e, (myokit.Plus, myokit.Minus)):
                 return self._sum(e)
-            if isinstance(e, myokit.Exp) and self._single and \
-                    not self._native:
+            if isinstance(e, myokit.Exp) and self._scale:
                 return self._scaled_exp(e[0])
         return super().ex(e)
 
@@ -199,9 +199,11 @@ class CudaExpressionWriter(CBasedExpressionWriter):
     def _scaled_exp(self, x):
         """
         exp(k X), k the literal factors of the argument, as
-        2^(X (k log2 e)): mkg_exp_scaled takes the factor in two parts.
+        2^(X (k log2 e)): mkg_exp_scaled takes the factor in two parts. It
+        is the more exact where the product k X would be rounded; without a
+        factor, or with a power of two, expf is.
         """
-        k = 1.0
+        k, argument = 1.0, x
         while True:
             if isinstance(x, myokit.PrefixMinus):
                 k, x = -k, x[0]
@@ -214,6 +216,8 @@ class CudaExpressionWriter(CBasedExpressionWriter):
                 k, x = k / float(x[1].eval()), x[0]
             else:
                 break
+        if abs(np.frexp(k)[0]) == 0.5:
+            return f'expf({self.ex(argument)})'
         return self.scaled_exp(self.ex(x), k)
 
     def scaled_exp(self, x, k):
@@ -447,7 +451,10 @@ _EXP_HELPER = '''
 // product against this: 3.9e-8 and 4.0e-8 for exponents near 0.2, 6.1e-8
 // and 6.2e-8 near 1.3, 1.7e-7 and 1.3e-7 near 5, 6.1e-7 and 3.9e-7 near 16;
 // largest errors 1.42e-7 and 1.37e-7, 2.6e-7 and 2.2e-7, 6.6e-7 and 4.7e-7,
-// 2.3e-6 and 1.4e-6.
+// 2.3e-6 and 1.4e-6. For fp32_math='fast' only, which flushes denormals, and
+// only where there is such a product: of an exact argument expf has 4.0e-8
+// at every exponent (largest error 1.5e-7), this 6.2e-8 near 1.3, 1.3e-7
+// near 5 and 3.9e-7 near 16 (2.2e-7, 4.6e-7 and 1.4e-6).
 static __device__ __forceinline__ Real mkg_exp_scaled(Real x, Real hi,
                                                       Real lo)
 {
@@ -826,7 +833,8 @@ class TissueKernel(object):
     def _generate(self):
         m = self.model
         w = CudaExpressionWriter(self.single, self.native_math,
-                                 self.math == 'fast', soft=True, fuse=True)
+                                 self.math == 'fast', soft=True, fuse=True,
+                                 scale=self.math == 'fast')
         w.set_lhs_function(self._name)
         real = 'float' if self.single else 'double'
         prec = myokit.SINGLE_PRECISION if self.single else \
@@ -1740,19 +1748,21 @@ class TissueKernel(object):
         """
         exp(-dt / tau) of a Rush-Larsen update: ``tau`` the time constant's
         text, ``var`` its variable. Where that is a reciprocal 1 / s the
-        exponent is -dt s, one division less.
+        exponent is -dt s, one division less (and in fast single precision
+        mkg_exp_scaled, whose rounding of it takes the place of the two of
+        the reciprocal and the quotient).
         """
         w = self.writer
         s = rates.get(var)
         if s is not None:
             x = f'dt_ * {w.ex(s)}'
+            if self.math == 'fast' and not self.native_math:
+                return w.scaled_exp(x, -1.0)
         elif self.single:
             x = f'dt_ / {tau}' if self.math != 'fast' else \
                 f'__fdividef(dt_, {tau})'
         else:
             x = w.divide('dt_', tau)
-        if self.single and not self.native_math:
-            return w.scaled_exp(x, -1.0)
         return f'{w._fn("exp")}(-({x}))'
 
     def _find_repeated(self):
