@@ -970,9 +970,12 @@ class SimulationCUDA(object):
         if res is not None:
             k = self._make_kernel(inter_log, mode, two_d, (32 * res[0], 1),
                                   res[1], res[0])
-            # (a model too large for that many tiles on an SM)
+            # (a model too large for that many tiles on an SM, which has 228
+            # KB and keeps one of them per CTA)
+            held = -(-k.resident_bytes() // 128) * 128 + 1024
             if k.resident_bytes() <= 48 * 1024 and \
-                    k.resident_bytes() * res[1] <= 216 * 1024:
+                    k.resident_bytes() * res[1] <= 216 * 1024 and \
+                    held * res[1] <= 228 * 1024:
                 return k
         block = self._block_shape(two_d)
         return self._make_kernel(inter_log, mode, two_d, block,
