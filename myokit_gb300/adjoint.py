@@ -806,9 +806,9 @@ class TissueAdjoint(object):
         kernel = sim._kernel([])
         be = sim._get_backend(kernel)
         # Generated once per forward kernel (the forward kernel's key covers
-        # the model version, precision, fields and launch shape)
-        akey = (kernel.key(), self.min_blocks, self.threads, self.guards,
-                self._tiles_per_sm(kernel))
+        # the model version, precision, fields and launch shape) and CTA size
+        akey = (kernel.key(), self.min_blocks, self._threads(kernel),
+                self.guards, self._tiles_per_sm(kernel))
         ak = self._generated.get(akey)
         if ak is None:
             ak = shared_kernel(
@@ -843,6 +843,21 @@ class TissueAdjoint(object):
         n = -(-(-(-nx // 32) * ny) // autotune._sm_count(sim._device))
         return n if n <= _MAP_TILES else 0
 
+    def _threads(self, kernel):
+        """The CTA size of the general reverse kernel."""
+        if self.threads is not None:
+            return self.threads
+        if kernel.team:
+            # A resident kernel's CTA is one tile; the reverse kernel's
+            # warps each own tiles: as many warps as there are tiles for an
+            # SM
+            return 32 * min(kernel.min_blocks, 8)
+        if self.sim._block is None:
+            # The reverse kernel wants the registers of 256 threads (800 x
+            # 800 cells, 48 states, 20 steps: 52.1 ms, with 512 53.3)
+            return min(kernel.block[0], 256)
+        return None
+
     def _make(self, kernel, tiles_per_sm):
         """The adjoint kernel of a forward kernel."""
         sim = self.sim
@@ -858,21 +873,12 @@ class TissueAdjoint(object):
             stage=kernel.stage, row_pad=kernel.row_pad,
             stage_lazy=kernel.stage_lazy, sync=kernel.sync,
             team=kernel.team)
-        threads = self.threads
         if tiles_per_sm:
             ak = AdjointKernel(fwd, tiles_per_sm=tiles_per_sm)
             if ak.parts:
                 return ak
-        if threads is None and kernel.team:
-            # A resident kernel's CTA is one tile; the reverse kernel's
-            # warps each own tiles: as many warps as there are tiles for an
-            # SM
-            threads = 32 * min(kernel.min_blocks, 8)
-        elif threads is None and sim._block is None:
-            # The reverse kernel wants the registers of 256 threads (800 x
-            # 800 cells, 48 states, 20 steps: 52.1 ms, with 512 53.3)
-            threads = min(kernel.block[0], 256)
-        return AdjointKernel(fwd, self.min_blocks, threads, self.guards)
+        return AdjointKernel(fwd, self.min_blocks, self._threads(kernel),
+                             self.guards)
 
     def forward(self, duration, log_interval=1.0):
         """
