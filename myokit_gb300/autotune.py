@@ -41,9 +41,11 @@ _CANDIDATES = [
     ((256, 1), 2, 0, True, _N),
     ((256, 1), 2, 0, 2, _B), ((384, 1), 1, 0, 2, _N),
 ]
+# (double precision: the shapes of default_shape among them)
 _CANDIDATES_FP64 = [((128, 1), 1, 0, False, _B), ((256, 1), 1, 0, False, _B),
                     ((64, 1), 1, 0, False, _B), ((32, 1), 1, 0, False, _B),
-                    ((256, 1), 1, 0, True, _B), ((256, 1), 1, 0, False, _N)]
+                    ((256, 1), 1, 0, True, _B), ((256, 1), 1, 0, False, _N),
+                    ((64, 1), 4, 0, True, _B), ((512, 1), 1, 0, True, _B)]
 # Grids with fewer warp tiles than SMs: teams of 2 to 16 warps share each
 # tile's work (a sixth entry: warps per tile): one team per CTA or two, or
 # one team per cluster of 2 or 4 CTAs
