@@ -952,9 +952,10 @@ class SimulationCUDA(object):
         if not all(x is None for x in (self._block, self._split, self._sync,
                                        self._stage_lazy, self._min_blocks)):
             return None
+        # (a choice that names no team was made among other shapes only)
         hit = self._tuned_choice()
-        if hit is not None:
-            if not hit.get('team'):
+        if hit is not None and 'team' in hit:
+            if not hit['team']:
                 return None
             return int(hit['team']), int(hit['min_blocks'])
         return autotune.resident_shape(

@@ -37,3 +37,30 @@ def test_candidates_hold_the_default_shape(decker, br77, empty_cache,
                     (c[5:] or (1,))[0] == 1))
                 for c in timed), (n, k.block, k.min_blocks)
             assert len(set(timed)) == len(timed)
+
+
+@pytest.mark.parametrize('saved,team', [
+    ({}, 4), ({'team': 0}, 0), ({'team': 2}, 2)])
+def test_choices_saved_before_there_were_resident_tiles(br77, empty_cache,
+                                                        saved, team):
+    # An entry that names no team was chosen among other shapes only: it
+    # does not keep a small grid off resident tiles. One that does stands
+    def new():
+        return mg.SimulationCUDA(br77, None, ncells=200)
+    entry = dict({'block': [128, 1], 'min_blocks': 1, 'steps_per_launch': 0,
+                  'stage_lazy': 0, 'sync': 'barrier', 'split': 4, 'rate': 1.0,
+                  'when': 'test'}, **saved)
+    if saved.get('team'):
+        entry.update(block=[64, 1], split=1)
+    with open(os.path.join(str(empty_cache), 'tune.json'), 'w') as f:
+        json.dump({at.signature(new()): entry}, f)
+    k = new()._kernel([])
+    assert k.team == team
+    if not team:
+        assert k.block == (128, 1) and k.split == 4
+    # Larger grids keep what was saved for them
+    s = mg.SimulationCUDA(br77, None, ncells=(512, 512))
+    with open(os.path.join(str(empty_cache), 'tune.json'), 'w') as f:
+        json.dump({at.signature(s): dict(entry, block=[384, 1], split=1)}, f)
+    if not saved.get('team'):
+        assert s._kernel([]).block == (384, 1)
