@@ -143,8 +143,8 @@ MKG_M64 double mkg_exp_fixed(mkg_u32 x2, mkg_u32 x1, mkg_u32 x0, mkg_u32 s)
 }
 
 /*
- * e^x, within 0.57 ulp (measured against long double; the library's
- * exp is specified to 1 ulp). Table-driven as in P.T.P. Tang, "Table-driven
+ * e^x, within 0.57 ulp on the device (CUDA's: 0.85, root mean square 0.301
+ * against 0.289 here; for |x| < 0.01 0.51, 0.2885 and 0.2887). Table-driven as in P.T.P. Tang, "Table-driven
  * implementation of the exponential function in IEEE floating-point
  * arithmetic" (ACM TOMS 15, 1989), in 64-bit fixed point:
  *   |x| as a fixed-point number, 64 bits after the point (exact for
@@ -322,15 +322,17 @@ MKG_M64 mkg_log_t mkg_log_fixed(mkg_u32 hx, mkg_u32 lx)
     return g;
 }
 
-/* Logarithm, within 0.52 ulp (the library's is specified to 1 ulp); where
- * it is below 2^-7 the library's function keeps the relative error */
+/* Logarithm, within 0.52 ulp (CUDA's: 0.54 measured, specified to 1); where
+ * its magnitude is below 2^-5 the library's function, which is the more exact
+ * there (0.501 ulp; the fixed point is off by 0.53 from 2^-6 and by 0.55 from
+ * 2^-7 on) */
 MKG_M64_FN double mkg_log(double x)
 {
     const mkg_u32 hx = mkg_hi(x);
     if (hx - 0x00100000u >= 0x7fe00000u) return mkg_log_slow(x);
     const mkg_log_t g = mkg_log_fixed(hx, mkg_lo(x));
     const mkg_u32 fh = (mkg_u32)(g.f >> 32), fl = (mkg_u32)g.f;
-    if (g.i == 0 ? fh < 0x02000000u : g.i > 0x7fffffffu)
+    if (g.i == 0 ? fh < 0x08000000u : g.i > 0x7fffffffu)
         return mkg_log_slow(x);
     /* The leading one to the top of 64 bits, 53 of them rounded */
     const mkg_u32 z = g.i ? mkg_clz(g.i) : mkg_clz(fh);
@@ -348,7 +350,7 @@ MKG_M64_FN double mkg_log(double x)
 /*
  * x^p for a literal p, 2^-8 <= |p| < 16: e^(p log x) with the product in
  * fixed point; P = |p| 2^60 (exact), neg all ones for p < 0. Within 0.6 ulp
- * (the library's pow is specified to 2 ulp).
+ * (CUDA's pow: 1.3).
  */
 MKG_M64_FN double mkg_pow_literal(double x, double p, mkg_u64 P, mkg_u32 neg)
 {
@@ -373,8 +375,8 @@ MKG_M64_FN double mkg_pow_literal(double x, double p, mkg_u64 P, mkg_u32 neg)
 /*
  * cos(acos(z) / 3), which cubic roots are written with: the root c in
  * [1/2, 1] of 4 c^3 - 3 c = z, by two Newton steps in fixed point from the
- * single precision value. Where the slope vanishes (z near -1) and outside
- * (-1, 1), the library's functions.
+ * single precision value, within 0.6 ulp (CUDA's functions: 2.0). Where the
+ * slope vanishes (z near -1) and outside (-1, 1), the library's functions.
  */
 MKG_M64_FN double mkg_cos_third(double z)
 {
