@@ -872,7 +872,7 @@ class TissueAdjoint(object):
             accumulate_states=sim.accumulated_states(), traj=True,
             stage=kernel.stage, row_pad=kernel.row_pad,
             stage_lazy=kernel.stage_lazy, sync=kernel.sync,
-            team=kernel.team)
+            team=kernel.team, many=kernel.many)
         if tiles_per_sm:
             ak = AdjointKernel(fwd, tiles_per_sm=tiles_per_sm)
             if ak.parts:

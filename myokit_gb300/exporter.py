@@ -684,7 +684,7 @@ class TissueKernel(object):
                  fast_divide=True, min_blocks=1, math='default',
                  accumulate=None, accumulate_states=(), traj=False,
                  stage=False, row_pad=False, stage_lazy=False,
-                 sync='barrier', split=1, team=0):
+                 sync='barrier', split=1, team=0, many=True):
         self.model = model
         self.single = (precision == myokit.SINGLE_PRECISION)
         self.native_math = bool(native_math)
@@ -758,6 +758,8 @@ class TissueKernel(object):
         self.team = int(team)
         if self.team not in (0, 1, 2, 4, 8, 16):
             raise ValueError('team must be 0, 1, 2, 4, 8 or 16')
+        # Connections: some cell has more than four (resident kernels)
+        self.many = bool(many) or not self.team
         if self.team:
             if self.block != (32 * self.team, 1) or self.split > 1:
                 raise ValueError('a resident tile is a CTA of its own')
@@ -1459,6 +1461,7 @@ class TissueKernel(object):
             '@TEAM@': str(self.team),
             '@NSLOT@': str(self.team_nslot),
             '@TRAJ@': '1' if self.traj else '0',
+            '@MANY@': '1' if self.many else '0',
             '@DEVICE@': _read('mkg_device.h'),
             '@FIELD_LOADS@': '\n'.join(
                 f'        if (part_ == {k % self.team}) fs[{k}][lane] = '

@@ -937,6 +937,19 @@ class SimulationCUDA(object):
                 out.append(st)
         return out
 
+    def _connection_arrays(self):
+        """
+        Cells and conductances of the connections, and the most that a cell
+        has (converted once per set_connections).
+        """
+        if self._c_arrays is None:
+            c = np.array(self._connections, dtype=float).reshape(-1, 3)
+            c1 = np.ascontiguousarray(c[:, 0].astype(np.int64))
+            c2 = np.ascontiguousarray(c[:, 1].astype(np.int64))
+            self._c_arrays = (c1, c2, np.ascontiguousarray(c[:, 2]), int(
+                np.bincount(np.concatenate([c1, c2]), minlength=1).max()))
+        return self._c_arrays
+
     def _resident(self, two_d):
         """
         ``(warps per tile, CTAs per SM)`` of a resident kernel, or None. By
@@ -958,6 +971,12 @@ class SimulationCUDA(object):
             if not hit['team']:
                 return None
             return int(hit['team']), int(hit['min_blocks'])
+        # (single precision steps are too short for the trips to L2 that
+        # more than about forty neighbours take, see MKG_MORE in the kernel)
+        if self._connections is not None and \
+                self._precision == myokit.SINGLE_PRECISION and \
+                self._connection_arrays()[3] > 40:
+            return None
         return autotune.resident_shape(
             tiles, autotune._sm_count(self._device),
             self._precision == myokit.SINGLE_PRECISION, self._nstate)
@@ -990,10 +1009,12 @@ class SimulationCUDA(object):
         row_pad = two_d and self._nx % 4 != 0
         lazy = 0 if team else stage and self._lazy_staging()
         split = 1 if team else self._split_mode()
+        many = not team or mode != _exp.DIFF_CONN or \
+            self._connection_arrays()[3] > 4
         key = (team,
             self._model_version, self._precision, self._native_math, mode,
             two_d, block, minb, self._fp32_math, self._accumulate,
-            stage, row_pad, lazy, self._sync_mode(), split,
+            stage, row_pad, lazy, self._sync_mode(), split, many,
             tuple(v.qname() for v in acc),
             tuple(v.qname() for v in self._fields.keys()),
             tuple(v.qname() for v in inter_log))
@@ -1009,7 +1030,8 @@ class SimulationCUDA(object):
                     min_blocks=minb, math=self._fp32_math,
                     accumulate=self._accumulate, accumulate_states=acc,
                     stage=stage, row_pad=row_pad, stage_lazy=lazy,
-                    sync=self._sync_mode(), split=split, team=team))
+                    sync=self._sync_mode(), split=split, team=team,
+                    many=many))
             if len(self._kernels) > 16:
                 self._kernels.clear()
             self._kernels[key] = k
@@ -1247,14 +1269,7 @@ class SimulationCUDA(object):
             be.check(lib.mkg_set_conductance_field(
                 h, _lib.dptr(gx), gx.size, _lib.dptr(gy), gy.size))
         elif mode == _exp.DIFF_CONN:
-            # Converted once per set_connections
-            if self._c_arrays is None:
-                c = np.array(self._connections, dtype=float).reshape(-1, 3)
-                self._c_arrays = (
-                    np.ascontiguousarray(c[:, 0].astype(np.int64)),
-                    np.ascontiguousarray(c[:, 1].astype(np.int64)),
-                    np.ascontiguousarray(c[:, 2]))
-            c1, c2, gg = self._c_arrays
+            c1, c2, gg, _ = self._connection_arrays()
             be.check(lib.mkg_set_connections(
                 h, _lib.i64ptr(c1), _lib.i64ptr(c2), _lib.dptr(gg), len(gg)))
         if not self._diffusion_enabled:
