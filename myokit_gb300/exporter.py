@@ -135,7 +135,7 @@ class CudaExpressionWriter(CBasedExpressionWriter):
     (``myokit/formats/opencl/_ewriter.py:59-93``).
     """
     def __init__(self, single, native_math=False, fast_divide=False,
-                 soft=False, fuse=False, scale=True):
+                 soft=False, fuse=False):
         super().__init__()
         self._single = bool(single)
         self._native = bool(native_math) and self._single
@@ -143,10 +143,9 @@ class CudaExpressionWriter(CBasedExpressionWriter):
         # Double precision exp and division in integer arithmetic
         # (csrc/mkg_math64.h)
         self._soft = bool(soft) and not self._single
-        # Multiply-adds and (scale) the scaling of single precision
-        # exponentials written out (see ex)
+        # Multiply-adds and the scaling of single precision exponentials
+        # written out (see ex)
         self._fuse = bool(fuse)
-        self._scale = bool(scale) and self._single and not self._native
         self.int_powers = set()
 
     # Kernels are compiled without the compiler's own contraction of
@@ -159,7 +158,8 @@ class CudaExpressionWriter(CBasedExpressionWriter):
         if self._fuse:
             if isinstance(e, (myokit.Plus, myokit.Minus)):
                 return self._sum(e)
-            if isinstance(e, myokit.Exp) and self._scale:
+            if isinstance(e, myokit.Exp) and self._single and \
+                    not self._native:
                 return self._scaled_exp(e[0])
         return super().ex(e)
 
@@ -451,15 +451,15 @@ _EXP_HELPER = '''
 // product against this: 3.9e-8 and 4.0e-8 for exponents near 0.2, 6.1e-8
 // and 6.2e-8 near 1.3, 1.7e-7 and 1.3e-7 near 5, 6.1e-7 and 3.9e-7 near 16;
 // largest errors 1.42e-7 and 1.37e-7, 2.6e-7 and 2.2e-7, 6.6e-7 and 4.7e-7,
-// 2.3e-6 and 1.4e-6. For fp32_math='fast' only, which flushes denormals, and
-// only where there is such a product: of an exact argument expf has 4.0e-8
-// at every exponent (largest error 1.5e-7), this 6.2e-8 near 1.3, 1.3e-7
-// near 5 and 3.9e-7 near 16 (2.2e-7, 4.6e-7 and 1.4e-6).
+// 2.3e-6 and 1.4e-6. Only where there is such a product: of an exact
+// argument expf has 4.0e-8 at every exponent (largest error 1.5e-7), this
+// 6.2e-8 near 1.3, 1.3e-7 near 5 and 3.9e-7 near 16 (2.2e-7, 4.6e-7 and
+// 1.4e-6). Denormals flush to zero with fp32_math='fast' alone.
 static __device__ __forceinline__ Real mkg_exp_scaled(Real x, Real hi,
                                                       Real lo)
 {
     float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaf(x, hi, x * lo)));
+    asm("ex2.approx@FTZ@.f32 %0, %1;" : "=f"(r) : "f"(fmaf(x, hi, x * lo)));
     return r;
 }'''
 
@@ -514,7 +514,7 @@ def cubic_root_coefficients(rhs):
     return None
 
 
-def _pow_helpers(single, outline=False):
+def _pow_helpers(single, outline=False, flush=False):
     """Inline helpers for x^n (n = 2..16, by repeated squaring) and x^1.5
     and, in single precision, the cubic root refinement."""
     out = []
@@ -543,8 +543,10 @@ def _pow_helpers(single, outline=False):
     out.append('static __device__ __forceinline__ Real mkg_pow1p5(Real x)'
                f' {{ return x * {sq}(x); }}')
     if single:
-        out.extend([_EXP_HELPER, _CUBIC_HELPER.replace(
-            '__forceinline__', '__noinline__') if outline else _CUBIC_HELPER])
+        out.extend([
+            _EXP_HELPER.replace('@FTZ@', '.ftz' if flush else ''),
+            _CUBIC_HELPER.replace('__forceinline__', '__noinline__')
+            if outline else _CUBIC_HELPER])
     return '\n'.join(out)
 
 
@@ -835,8 +837,7 @@ class TissueKernel(object):
     def _generate(self):
         m = self.model
         w = CudaExpressionWriter(self.single, self.native_math,
-                                 self.math == 'fast', soft=True, fuse=True,
-                                 scale=self.math == 'fast')
+                                 self.math == 'fast', soft=True, fuse=True)
         w.set_lhs_function(self._name)
         real = 'float' if self.single else 'double'
         prec = myokit.SINGLE_PRECISION if self.single else \
@@ -1152,7 +1153,8 @@ class TissueKernel(object):
             '@BX@': str(self.block[0]),
             '@BY@': str(self.block[1]),
             '@MINB@': str(self.min_blocks),
-            '@POW_HELPERS@': _pow_helpers(self.single),
+            '@POW_HELPERS@': _pow_helpers(
+                self.single, flush=self.math == 'fast'),
             '@LOADS@': '\n'.join(loads + field_loads),
             '@LOG_A@': log_a,
             '@BODY@': '\n'.join(body),
@@ -1482,7 +1484,8 @@ class TissueKernel(object):
             # and 2.4, one tile 2.49 and 2.51.
             '@POW_HELPERS@': '\n'.join([_pow_helpers(
                 self.single, not self.single or
-                self.team > 1 and len(self.cubic) > 1)] + self.functions),
+                self.team > 1 and len(self.cubic) > 1,
+                self.math == 'fast')] + self.functions),
             '@NEED_HALO@': ' || '.join(f'part_ == {p}' for p in halo)
             or 'false',
                     }
@@ -1751,7 +1754,7 @@ class TissueKernel(object):
         """
         exp(-dt / tau) of a Rush-Larsen update: ``tau`` the time constant's
         text, ``var`` its variable. Where that is a reciprocal 1 / s the
-        exponent is -dt s, one division less (and in fast single precision
+        exponent is -dt s, one division less (and in single precision
         mkg_exp_scaled, whose rounding of it takes the place of the two of
         the reciprocal and the quotient).
         """
@@ -1759,7 +1762,7 @@ class TissueKernel(object):
         s = rates.get(var)
         if s is not None:
             x = f'dt_ * {w.ex(s)}'
-            if self.math == 'fast' and not self.native_math:
+            if self.single and not self.native_math:
                 return w.scaled_exp(x, -1.0)
         elif self.single:
             x = f'dt_ / {tau}' if self.math != 'fast' else \
@@ -1895,7 +1898,8 @@ class FiberTissueKernel(object):
             '@SINGLE@': '1' if self.single else '0',
             '@BX@': str(self.block[0]),
             '@MINB@': str(self.min_blocks),
-            '@POW_HELPERS@': _pow_helpers(self.single),
+            '@POW_HELPERS@': _pow_helpers(
+                self.single, flush=fiber.math == 'fast'),
         }
         for name, k in (('FIBER', fiber), ('TISSUE', tissue)):
             for part in ('loads', 'log_a', 'body', 'log_b'):

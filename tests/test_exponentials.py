@@ -1,8 +1,8 @@
 """
 Single precision exponentials: 2^t with the argument's literal factor in two
-parts only where ``fp32_math='fast'`` and that factor would be rounded with
-the argument; else the library's function, which is within an ulp at any
-exponent and keeps denormals in the modes that promise to.
+parts only where their product would be rounded; else the library's function,
+which is within an ulp at any exponent. Denormals are kept in the modes that
+promise to.
 """
 import numpy as np
 import pytest
@@ -41,12 +41,13 @@ def _texts(model, math):
 def test_which_exponentials_are_scaled(br77, math):
     k, text = _texts(br77, math)
     scaled = [t.startswith('mkg_exp_scaled(') for t in text]
-    assert scaled == [False] * 5 + [math == 'fast'] * 2
+    assert scaled == [False] * 5 + [True] * 2
     assert all(t.startswith('expf(') for t, x in zip(text, scaled) if not x)
-    if math != 'fast':
-        # (the helper's own line is the only one left)
-        assert k.source().count('mkg_exp_scaled(') == 1
-        assert '--ftz=false' in k.options()
+    # Flushing denormals in fast mode only
+    flush = math == 'fast'
+    assert ('ex2.approx.ftz.f32' in k.source()) == flush
+    assert ('ex2.approx.f32' in k.source()) != flush
+    assert ('--ftz=true' in k.options()) == flush
 
 
 @pytest.mark.parametrize('math', ['fast', 'default', 'ieee'])
@@ -57,7 +58,7 @@ def test_decay_of_gates(decker, math):
     assert k.rl_states
     for inf, tau in k.rl_states.values():
         t = k.decay(tau, k._name(tau), k.rates)
-        scaled = math == 'fast' and tau in k.rates
+        scaled = tau in k.rates
         assert t.startswith('mkg_exp_scaled(' if scaled else 'expf(-(')
 
 
