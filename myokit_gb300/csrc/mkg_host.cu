@@ -1966,6 +1966,17 @@ int adj_attach(mkg_sim *s, const void *cubin, size_t size,
 {
     if (!s || !cubin || !size) return set_err(s, MKG_ERR_ARG, "null argument");
     if (seg_steps < 1) return set_err(s, MKG_ERR_ARG, "seg_steps < 1");
+    /* Nothing is attached until all of it is, and no forward run counts that
+     * was made with other kernels and buffers */
+    s->adj_seg = 0;
+    s->traj_segment = -1;
+    s->tape_steps = 0;
+    s->adj_rows = 0;
+    s->adj_sched.clear();
+    s->adj_seg_start.clear();
+    s->adj_seg_len.clear();
+    s->adj_seg_vsel.clear();
+    s->adj_log.clear();
     if (s->adj_lib) {
         cudaLibraryUnload(s->adj_lib);
         s->adj_lib = nullptr;
@@ -2034,10 +2045,7 @@ int adj_attach(mkg_sim *s, const void *cubin, size_t size,
     CK(s, cudaMalloc((void **)&s->d_probe_col, s->pitch * sizeof(int)));
     CK(s, cudaMalloc((void **)&s->d_fsteps, seg_steps * sizeof(mkg_step)));
     CK(s, cudaMalloc((void **)&s->d_bsteps, seg_steps * sizeof(mkg_step)));
-    s->adj_seg = seg_steps;
-    s->traj_segment = -1;
     dfree(s->d_tape);
-    s->tape_steps = 0;
     if (slots) {
         const size_t step = (size_t)tiles * slots * 32 * s->real;
         long long n = std::min<long long>(
@@ -2053,6 +2061,7 @@ int adj_attach(mkg_sim *s, const void *cubin, size_t size,
         CK(s, e);
         s->tape_steps = n;
     }
+    s->adj_seg = seg_steps;
     return MKG_OK;
 }
 
@@ -2078,7 +2087,7 @@ extern "C" int mkg_adj_forward(mkg_sim *s, double tmin, double tmax,
                                int64_t *rows_out)
 {
     if (!s) return set_err(s, MKG_ERR_ARG, "null argument");
-    if (!s->adj_lib) return set_err(s, MKG_ERR_ORDER, "mkg_adj_attach first");
+    if (!s->adj_seg) return set_err(s, MKG_ERR_ORDER, "mkg_adj_attach first");
     int r = mkg_run_begin(s, tmin, tmax, dt, log_interval);
     if (r) return r;
     s->adj_sched.clear();
@@ -2487,7 +2496,7 @@ extern "C" int mkg_adj_backward(mkg_sim *s, const double *lgrad,
                                 double *grad_g)
 {
     if (!s) return set_err(s, MKG_ERR_ARG, "null argument");
-    if (!s->adj_lib) return set_err(s, MKG_ERR_ORDER, "mkg_adj_attach first");
+    if (!s->adj_seg) return set_err(s, MKG_ERR_ORDER, "mkg_adj_attach first");
     if (rows != s->adj_rows)
         return set_err(s, MKG_ERR_ARG, "expected %lld rows",
                        (long long)s->adj_rows);
