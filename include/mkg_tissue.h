@@ -294,6 +294,8 @@ int mkg_last_stats(const mkg_sim *sim, double *kernel_ms, int64_t *launches,
  * ones, and mkg_adj_conductance_gradient then gives each edge's gradient.
  * With an accumulation mode the forward and its recomputation run as the
  * simulation's own kernel; the reverse sweep runs in the kernel precision.
+ * An attachment forgets the forward run made with the last one; one that
+ * fails leaves nothing attached (MKG_ERR_ORDER from the others).
  */
 int mkg_adj_attach(mkg_sim *sim, const void *cubin, size_t size,
                    int32_t seg_steps);

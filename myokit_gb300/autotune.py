@@ -154,7 +154,14 @@ def default_shape(single, n_state, plane_bytes, tiles_per_sm):
       against 20.7, Kahan 22.4 and 22.6, per-edge 23.1 and 23.9, FP64
       accumulation 41.4 and 43.0; 8 states 640 x 520 8.0 and 8.2, 512 x 512
       6.4 and 7.1, 290 x 290 4.0 and 4.7: their steps are too short to hide
-      the neighbours' counters);
+      the neighbours' counters). With many states neither is always ahead
+      there: barrier and neighbours, plain, Kahan, FP64 accumulation and
+      per-edge, 256 x 256 7.3 and 7.4, 8.0 and 8.3, 13.9 and 14.1, 7.5 and
+      7.7; 320 x 320 11.3 and 10.9, 12.3 and 12.1, 20.4 and 19.9, 11.7 and
+      11.3; 400 x 400 16.0 and 15.5, 17.4 and 17.5, 30.3 and 30.4, 16.5 and
+      16.3; 448 x 448 17.5 and 16.7, 19.1 and 18.3, 33.6 and 33.1, 18.0 and
+      17.4; 512 x 512 20.9 and 20.8, 22.7 and 23.1, 42.2 and 42.6, 21.5 and
+      21.7;
     - double precision, many states: 8 warps per SM of 64-thread CTAs, read
       from shared memory where used: 256 x 256 114 against 180 with 128
       threads and prefetch, 301 x 211 119 and 182, 512 x 512 491 and 676;

@@ -9,15 +9,15 @@
  * 32 x 32 -> 64 multiply-add every two to four). The library's exp is some
  * twenty double precision instructions and its division eight, so in a cell
  * model they are most of a step's time. Here both run on the integer pipes:
- * about 75 and 65 instructions, and no double precision one. Arguments
- * outside the common range go to the library's function.
+ * about 75 and 65 instructions, and no double precision one; the others
+ * likewise. Arguments outside the common range go to the library's function.
  *
- * Measured (one time step, launch shape unchanged): a 200-cell Beeler-Reuter
- * cable 24.2 -> 13.8 us (153 double precision instructions per cell instead
- * of about 720), a 256 x 256 sheet of a 48-state model 457 -> 218 us (1030
- * instead of about 4200; 27 thousand instructions in all, a fifth of the
- * issue slots: what is left waits for the double precision pipe and for the
- * two warps per scheduler that 194 registers allow).
+ * Measured (one time step): with exp and division alone, the launch shape
+ * unchanged, a 200-cell Beeler-Reuter cable 24.2 -> 13.8 us, a 256 x 256
+ * sheet of a 48-state model 457 -> 218 us. With all of them, and the tile of
+ * the cable and the launch shape of the sheet as they are by default now, 2.4
+ * and 115 us: 153 double precision instructions per tile and step instead of
+ * 727, and 660 instead of 2900; the sheet's step has 25,000 integer ones.
  *
  * The tables mkg_exp_tab and mkg_log_tab are written by the exporter.
  */
