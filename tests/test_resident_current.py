@@ -30,6 +30,22 @@ def _balances(model, n):
     return m
 
 
+def _through(model):
+    """``model`` with two states that the current reaches through others."""
+    m = model.clone()
+    i = m.binding('diffusion_current').qname()
+    c = m.add_component('through')
+    x = [c.add_variable('x%d' % q) for q in range(2)]
+    for v in x:
+        v.set_rhs('0')
+        v.promote(1.0)
+    c.add_variable('t').set_rhs('%s + 0.5 * through.x0' % i)
+    c.add_variable('e').set_rhs('exp(-0.0001 * through.t * through.t)')
+    x[0].set_rhs('-0.001 * (through.t + through.e)')
+    x[1].set_rhs('-0.01 * through.e * through.x1')
+    return m
+
+
 def _parts(k):
     """Each warp's code of a step, cut where the team meets."""
     body = re.split(r'\n *(?:else )?if \(part_ == \d+\) \{\n',
@@ -70,6 +86,16 @@ def test_current_is_read_before_it_changes(decker, br77, team, n, precision,
         k = _kernel(_balances(m, n), precision, team, rl, **kw)
         _check_plan(k)
         assert _check_current(k) >= 1
+
+
+@pytest.mark.parametrize('precision', [SP, DP])
+@pytest.mark.parametrize('team', [2, 4, 8])
+def test_current_through_other_variables(decker, br77, team, precision):
+    for m, rl in ((decker, True), (br77, False)):
+        k = _kernel(_through(m), precision, team, rl)
+        _check_plan(k)
+        _check_current(k)
+        _check_stop(k)
 
 
 def test_current_of_default_launch_shapes(decker, br77):
@@ -134,11 +160,15 @@ def test_several_balances_equal_undivided(decker, br77, precision, kw):
             (br77, False, 150, dict(conn=near)),
             (br77, False, (41, 7), dict(hetero=True)),
             (decker, True, (61, 5), {})):
-        m = _balances(m, 2)
-        one = 0 if isinstance(shape, tuple) else ''
-        log = ['%s3.balance.x1' % ('' if one == '' else '2.')]
-        want = _run(m, 0, shape, precision, rl, log=log, **more, **kw)
-        assert not np.all(want[1][log[0]] == 1.0)
-        for team in (2, 4, 8, 4, 2):
-            _same(want, _run(m, team, shape, precision, rl, log=log, **more,
-                             **kw))
+        for m, name in ((_balances(m, 2), 'balance.x1'),
+                        (_through(m), 'through.x1')):
+            _check_runs(m, rl, shape, more, precision, kw, name)
+
+
+def _check_runs(m, rl, shape, more, precision, kw, name):
+    log = ['%s3.%s' % ('2.' if isinstance(shape, tuple) else '', name)]
+    want = _run(m, 0, shape, precision, rl, log=log, **more, **kw)
+    assert not np.all(want[1][log[0]] == 1.0)
+    for team in (2, 4, 8, 4, 2):
+        _same(want, _run(m, team, shape, precision, rl, log=log, **more,
+                         **kw))
